@@ -81,7 +81,7 @@ __global__ void __launch_bounds__(128) k_adj_entries(AdjEntryArgs a, unsigned lo
             const int64_t di = ci - i, dj = cj - j;
             double cube;
             if (di >= -1 && di <= 1 && dj >= -1 && dj <= 1)
-                cube = a.acube[ij * 9 + 3 * (dj + 1) + (di + 1)];
+                cube = a.acube[ij + (3 * (dj + 1) + (di + 1)) * nxy];
             else
             {
                 const double rr = al / a.alpha[n];

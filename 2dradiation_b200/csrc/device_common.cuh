@@ -38,8 +38,8 @@
 //   rk fields    rkf[ij * kRkStride + f]  node-major pack of the 21 metric arrays
 //                                         the geodesic right-hand side reads and
 //                                         the 2x2 spatial tetrad blocks
-//   alpha cubes  acube[ij * 9 + 3(dj+1) + (di+1)] = (alpha_ij / alpha_n)^3 for
-//                                         the 3x3 neighbours n of interior ij
+//   alpha cubes  acube[(3(dj+1) + (di+1)) * nxy + ij] = (alpha_ij / alpha_n)^3
+//                                         for the 3x3 neighbours n of interior ij
 #pragma once
 #include <cuda.h>
 #include <cuda_runtime.h>

@@ -43,45 +43,47 @@ __device__ __forceinline__ double stream_value(const PlainStepArgs &a, int d, co
         int g0 = (unsigned)gz < (unsigned)a.ng ? gz : gz % a.ng;
         g0 = g0 < 0 ? 0 : g0;
         const int g1 = g0 + 1 == a.ng ? 0 : g0 + 1; // (g0 + 1) % nGrid
-        const double t = r.z - (double)g0;
-        const IgRow R0 = a.ig_rows[g0], R1 = a.ig_rows[g1];
-        const int idx0[4] = {R0.idx.x, R0.idx.y, R0.idx.z, R0.idx.w};
-        const int idx1[4] = {R1.idx.x, R1.idx.y, R1.idx.z, R1.idx.w};
-        const double w0[4] = {R0.w01.x, R0.w01.y, R0.w23.x, R0.w23.y};
-        const double w1[4] = {R1.w01.x, R1.w01.y, R1.w23.x, R1.w23.y};
+        // Each row is 4 consecutive directions, and the next row starts at
+        // the same one or one further on (checked for every direction count
+        // in tests/test_plain_paths.py): the two rows read 5 directions.
+        const double t = r.z - (double)g0, t1 = 1.0 - t;
+        const IgRow *r0 = a.ig_rows + g0, *r1 = a.ig_rows + g1;
+        const int b0 = __ldg(&r0->idx.x);
+        const bool shift = __ldg(&r1->idx.x) != b0;
+        const double2 wa = __ldg(&r0->w01), wb = __ldg(&r0->w23), wc = __ldg(&r1->w01), wd = __ldg(&r1->w23);
         const double al = __ldg(a.alpha + ij);
-        // element offsets of the 8 rows' planes
-        Off o0[4], o1[4];
+        const int n00 = i0 + j0 * nx;
+        Off o[5]; // element offsets of the directions at corner 00
 #pragma unroll
-        for (int k = 0; k < 4; k++)
+        for (int k = 0; k < 5; k++)
         {
-            o0[k] = (Off)idx0[k] * (Off)nxy;
-            o1[k] = (Off)idx1[k] * (Off)nxy;
+            const int dk = b0 + k;
+            o[k] = (Off)(dk >= a.nd ? dk - a.nd : dk) * (Off)nxy + (Off)n00;
         }
+        const int di0 = i0 - (int)i, dj0 = j0 - (int)j;
+        const bool near = di0 >= -1 && di0 <= 0 && dj0 >= -1 && dj0 <= 0;
+        const double *cube00 = a.acube + (ij + (int64_t)(3 * (dj0 + 1) + (di0 + 1)) * nxy);
         double Iq[4];
 #pragma unroll
         for (int q = 0; q < 4; q++) // corners 00, 01, 10, 11
         {
-            const int ci = i0 + (q >> 1), cj = j0 + (q & 1);
-            const int n = ci + cj * nx;
-            double v0 = 0.0, v1 = 0.0;
-#pragma unroll
-            for (int k = 0; k < 4; k++)
-            {
-                v0 += w0[k] * __ldg(a.Iin + (o0[k] + (Off)n));
-                v1 += w1[k] * __ldg(a.Iin + (o1[k] + (Off)n));
-            }
-            double v = v0 * (1.0 - t) + v1 * t;
+            const int off = (q >> 1) + (q & 1) * nx;
+            const double x0 = __ldg(a.Iin + (o[0] + (Off)off)), x1 = __ldg(a.Iin + (o[1] + (Off)off));
+            const double x2 = __ldg(a.Iin + (o[2] + (Off)off)), x3 = __ldg(a.Iin + (o[3] + (Off)off));
+            const double x4 = __ldg(a.Iin + (o[4] + (Off)off));
+            const double y0 = shift ? x1 : x0, y1 = shift ? x2 : x1, y2 = shift ? x3 : x2, y3 = shift ? x4 : x3;
+            const double v0 = wa.x * x0 + wa.y * x1 + wb.x * x2 + wb.y * x3;
+            const double v1 = wc.x * y0 + wc.y * y1 + wd.x * y2 + wd.y * y3;
+            double v = v0 * t1 + v1 * t;
             if (!(0.0 < v))
                 clamp_mask &= ~(1u << q);
             v = (0.0 < v) ? v : 0.0;
-            const int di = ci - (int)i, dj = cj - (int)j;
             double cube;
-            if (di >= -1 && di <= 1 && dj >= -1 && dj <= 1)
-                cube = __ldg(a.acube + ij * 9 + 3 * (dj + 1) + (di + 1));
+            if (near)
+                cube = __ldg(cube00 + (int64_t)((q >> 1) + 3 * (q & 1)) * nxy);
             else
             {
-                const double rr = al / __ldg(a.alpha + n);
+                const double rr = al / __ldg(a.alpha + n00 + off);
                 cube = rr * (rr * rr);
             }
             Iq[q] = cube * v;
@@ -157,12 +159,13 @@ __device__ __forceinline__ double collide_value(double I, double n1, double n2, 
 // half an ulp of 1/den and q within one ulp of num/den, the remainder
 // num - den q is exact in one fma and RN(q + rem r) is the correctly rounded
 // quotient) gives the IEEE result.  Used where den is the same for many
-// divisions; outside the range in which no step can underflow or overflow
-// the ordinary division is taken.  Requires 1 <= den < 2^100.
+// divisions; outside 2^-900 <= |num| < 2^900, where a step could underflow or
+// overflow, the ordinary division is taken.  Requires 1 <= den < 2^100.
 __device__ __forceinline__ double div_rn(double num, double den, double r)
 {
-    const double an = fabs(num);
-    if (an != 0.0 && !(an > 0x1p-900 && an < 0x1p+900))
+    // exponent field in [123, 1923) or exactly zero, tested on the integer pipe
+    const unsigned hi = (unsigned)__double2hiint(num), ex = (hi >> 20) & 0x7ffu;
+    if (ex - 123u >= 1800u && ((hi << 1) | (unsigned)__double2loint(num)) != 0u)
         return num / den;
     double q = __dmul_rn(num, r);
     q = __fma_rn(__fma_rn(-q, den, num), r, q);
@@ -306,131 +309,6 @@ __device__ __forceinline__ double stream_value_adaptive(const PlainStepArgs &a, 
 // any result.  ADAPTIVE: the adaptive streaming types -- each cell's stencil
 // is rotated by its new angle (its directions in stream, moments and
 // collide) and corners are read in their previous frames.
-//
-// Direction d of a cell's stencil (tn1, tn2: the stencil's directions;
-// rotated by the cell's angle in adaptive streaming).
-#define GRLBM_N1(d) (ADAPTIVE ? tn1[d] * rot_c - tn2[d] * rot_s : tn1[d])
-#define GRLBM_N2(d) (ADAPTIVE ? tn1[d] * rot_s + tn2[d] * rot_c : tn2[d])
-
-// The rest of a step for one cell once its streamed values are known: m
-// holds their moments; Sin points at them (direction stride sst), Sout at the
-// cell's output slots (the same slots in the fused step).  Collide
-// (src/Radiation.cpp:641-736) for a colliding cell, then the stored moments
-// and the lambda-iteration statistics.
-// tw, tn1, tn2: the stencil's weights and directions (global or shared memory).
-// rot_s, rot_c: the cell's rotation (adaptive streaming).
-// Unroll of the lambda iteration's direction loops for a fluid at rest (the
-// directions' updates are independent; only the moment sums chain them).
-#ifndef GRLBM_ITER_UNROLL
-#define GRLBM_ITER_UNROLL 4
-#endif
-constexpr int kIterUnroll = GRLBM_ITER_UNROLL;
-template <bool RECORD, bool ADAPTIVE>
-__device__ __forceinline__ void finish_cell(const PlainStepArgs &a, const StepRecord &rec, bool active, bool collides,
-                                            int64_t ij, int64_t cc, Moments m, const double *Sin, int64_t sst,
-                                            double *Sout,
-                                            double rot_s, double rot_c, const double *tw, const double *tn1,
-                                            const double *tn2)
-{
-    const int t = threadIdx.x;
-    const int64_t nxy = a.g.nxy;
-    int cycles = 0;
-    if (RECORD && active)
-        rec.e0[cc] = m.E;
-    if (collides)
-    {
-        const double u1 = a.u1[ij], u2 = a.u2[ij], lor = a.lor[ij], adt = a.adt[ij];
-        const double eta = a.eta[ij], k0 = a.k0[ij], k3 = a.k3[ij], kak0 = a.ka[ij] + a.k0[ij];
-        // A fluid at rest has u = 0 and lorentz = 1, so in collide_value
-        // A = 1, n_ff = n and AA = 1 exactly: the update reduces to
-        // (I + adt (eta + (k0 fE + k3 (n1 fFx + n2 fFy)))) / (1 + adt kak0)
-        // with the same roundings.
-        const bool rest = u1 == 0.0 && u2 == 0.0 && lor == 1.0;
-        const double den = 1.0 + adt * kak0;
-        const bool fast_div = rest && den >= 1.0 && den < 0x1p+100;
-        const double rden = __drcp_rn(den);
-        double diff = 1;
-        double fE = 0, fFx = 0, fFy = 0;
-        while (fabs(diff) > 1e-4 && cycles < 100)
-        {
-            cycles++;
-            const double pE = m.E, pFx = m.Fx, pFy = m.Fy, pPxx = m.Pxx, pPxy = m.Pxy, pPyy = m.Pyy;
-            // fluid-frame moments of the previous iterate (src/Radiation.cpp:672-678)
-            const double uF = u1 * pFx + u2 * pFy;
-            const double uxP = u1 * pPxx + u2 * pPxy;
-            const double uyP = u1 * pPxy + u2 * pPyy;
-            const double uuP = u1 * uxP + u2 * uyP;
-            fE = lor * lor * (pE - 2.0 * uF + uuP);
-            fFx = lor * lor * (pFx - lor * pE * u1 - uxP + u1 * lor / (1.0 + lor) * ((2.0 * lor + 1.0) * uF - lor * uuP));
-            fFy = lor * lor * (pFy - lor * pE * u2 - uyP + u2 * lor / (1.0 + lor) * ((2.0 * lor + 1.0) * uF - lor * uuP));
-            m.zero();
-            if (rest)
-            {
-                const double k0fE = k0 * fE;
-#pragma unroll kIterUnroll
-                for (int d = 0; d < a.nd; d++)
-                {
-                    const double n1 = GRLBM_N1(d), n2 = GRLBM_N2(d);
-                    const double num = Sin[(int64_t)d * sst] + adt * (eta + (k0fE + k3 * (n1 * fFx + n2 * fFy)));
-                    const double v = fast_div ? div_rn(num, den, rden) : num / den;
-                    m.add(tw[d], v, n1, n2);
-                }
-            }
-            else
-                for (int d = 0; d < a.nd; d++)
-                {
-                    const double n1 = GRLBM_N1(d), n2 = GRLBM_N2(d);
-                    const double v = collide_value(Sin[(int64_t)d * sst], n1, n2, u1, u2, lor, adt, eta, k0, k3,
-                                                   kak0, fE, fFx, fFy);
-                    m.add(tw[d], v, n1, n2);
-                }
-            const double e1 = (pE - m.E) / m.E, e2 = (pFx - m.Fx) / m.Fx, e3 = (pFy - m.Fy) / m.Fy;
-            const double e4 = (pPxx - m.Pxx) / m.Pxx, e5 = (pPxy - m.Pxy) / m.Pxy, e6 = (pPyy - m.Pyy) / m.Pyy;
-            diff = sqrt(e1 * e1 + e2 * e2 + e3 * e3 + e4 * e4 + e5 * e5 + e6 * e6);
-        }
-        // the last iterate, recomputed from the same operands, over the parked values
-        if (rest)
-        {
-            const double k0fE = k0 * fE;
-#pragma unroll kIterUnroll
-            for (int d = 0; d < a.nd; d++)
-            {
-                const double n1 = GRLBM_N1(d), n2 = GRLBM_N2(d);
-                const double num = Sin[(int64_t)d * sst] + adt * (eta + (k0fE + k3 * (n1 * fFx + n2 * fFy)));
-                Sout[(int64_t)d * nxy] = fast_div ? div_rn(num, den, rden) : num / den;
-            }
-        }
-        else
-            for (int d = 0; d < a.nd; d++)
-                Sout[(int64_t)d * nxy] = collide_value(Sin[(int64_t)d * sst], GRLBM_N1(d), GRLBM_N2(d), u1, u2,
-                                                     lor, adt, eta, k0, k3, kak0, fE, fFx, fFy);
-    }
-    if (RECORD && active)
-        rec.cycles[cc] = cycles;
-    if (active)
-    {
-        a.mom[ij] = m.E;
-        a.mom[ij + nxy] = m.Fx;
-        a.mom[ij + 2 * nxy] = m.Fy;
-        a.mom[ij + 3 * nxy] = m.Pxx;
-        a.mom[ij + 4 * nxy] = m.Pxy;
-        a.mom[ij + 5 * nxy] = m.Pyy;
-    }
-    // lambda-iteration statistics: warp sums and maxima, one atomic per warp
-    unsigned sum = (unsigned)cycles, mx = (unsigned)cycles;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1)
-    {
-        sum += __shfl_xor_sync(0xffffffffu, sum, o);
-        mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-    }
-    if ((t & 31) == 0 && sum)
-    {
-        atomicAdd(a.iter_sum, (unsigned long long)sum);
-        atomicMax(a.iter_max, mx);
-    }
-}
-
 
 // The fixed streaming types run the step as two kernels, so that the
 // stream's dependent gathers (record, interpolation rows, 32 corner taps)
@@ -440,10 +318,6 @@ __device__ __forceinline__ void finish_cell(const PlainStepArgs &a, const StepRe
 // clamp mask).
 // Blocks are 32 x 4 tiles of cells (blockIdx.x, blockIdx.y over the slab
 // rows) of one direction (blockIdx.z).
-#ifndef GRLBM_COLLIDE_UNROLL
-#define GRLBM_COLLIDE_UNROLL 8
-#endif
-constexpr int kCollideUnroll = GRLBM_COLLIDE_UNROLL;
 // Grid order of the stream kernel: directions fastest for adaptive streaming
 // (the blocks of one tile, which read the same Fourier coefficients, run
 // together), tiles fastest for fixed streaming (measured: 2% faster and 3%
@@ -492,6 +366,165 @@ __global__ void __launch_bounds__(kStepBlock, GRLBM_STREAM_MIN_BLOCKS) k_stream_
     a.S[(int64_t)d * a.g.nxy + ij] = val;
 }
 
+// Curved fixed stream from a staged patch: a block takes 16 x 4 cells with
+// all their directions.  It first copies the state of the tile's 18 x 6 nodes
+// ([direction][row][node], nd * 896 bytes) and its cells' alpha cubes into
+// shared memory; its threads (64 cells x 4 directions at a time) then stream
+// direction after direction, each thread's next record loaded while the
+// current one is worked on.  Same arithmetic, in the same order, as
+// stream_value<true>.
+//
+// What bounds the gather from global memory (stream_value) is latency: record,
+// interpolation rows and 20 corner taps one after the other at 24 warps per
+// SM (266 us at 400^2 x 64, DRAM 21% and L1 62% busy; fewer tap loads and
+// coalesced alpha cubes alone left it at 270 us).  Here a tap is a
+// conflict-free 8-byte shared-memory read and only the record still comes
+// from DRAM, a direction ahead.
+constexpr int kPatchX = 16, kPatchY = 4;
+constexpr int kPatchCells = kPatchX * kPatchY;
+// (a direction's plane is a multiple of 16 doubles: lanes whose windows start
+// at different directions still read the banks of their own nodes)
+constexpr int kPatchPitch = kPatchX + 2, kPatchNodes = kPatchPitch * (kPatchY + 2);
+constexpr int kPatchPlane = (kPatchNodes + 15) / 16 * 16;
+// with more directions the patch and its rows leave one block per SM: those
+// gather from global memory
+constexpr int kPatchMaxDirs = 88;
+// up to this three blocks of 4 directions fit an SM, above it two of 6: 24
+// warps of 80 registers either way (200^2 x 32: 21.8 us against 23.7; 400^2 x
+// 64: 149 us against 140)
+constexpr int kPatchFewDirs = 57;
+__host__ __device__ constexpr size_t patch_smem(int nd)
+{
+    return ((size_t)nd * kPatchPlane + 9 * kPatchCells) * sizeof(double) + (size_t)10 * nd * 36;
+}
+__device__ __forceinline__ void copy8_async(double *dst, const double *src)
+{
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src)
+                 : "memory");
+}
+__device__ __forceinline__ double4 load_once(const double4 *p)
+{
+    const double2 lo = __ldcs(reinterpret_cast<const double2 *>(p)), hi = __ldcs(reinterpret_cast<const double2 *>(p) + 1);
+    return make_double4(lo.x, lo.y, hi.x, hi.y);
+}
+template <bool RECORD, int DIRS>
+__global__ void __launch_bounds__(kPatchCells * DIRS, DIRS == 4 ? 3 : 2)
+    k_stream_plain_patch(const __grid_constant__ PlainStepArgs a, const __grid_constant__ StepRecord rec)
+{
+    // [d][row][node], the cells' 9 alpha cubes [n][cell], the interpolation rows
+    extern __shared__ double patch[];
+    constexpr int kPatchDirs = DIRS, kPatchThreads = kPatchCells * DIRS;
+    const int t = threadIdx.x, lx = t % kPatchX, ly = (t / kPatchX) % kPatchY, dg = t / kPatchCells;
+    const int cell = t % kPatchCells;
+    const int nx = (int)a.g.nx, nd = a.nd;
+    const int x0 = (int)blockIdx.x * kPatchX, y0 = (int)a.g.jlo - 1 + (int)blockIdx.y * kPatchY; // the patch's first node
+    const int64_t nxy = a.g.nxy;
+    double *cubes = patch + (size_t)nd * kPatchPlane;
+    const int i = 1 + x0 + lx, j = 1 + y0 + ly;
+    const bool active = i <= (int)a.g.nx_ && j < (int)a.g.jhi;
+    const int ij = i + j * nx;
+    const int64_t cc = (int64_t)(i - 1) + (int64_t)(j - 1) * a.g.nx_;
+    const bool streams = active && !(a.flags[ij] & 2);
+    double4 r = make_double4(0, 0, 0, 0);
+    if (streams && dg < nd)
+        r = load_once(a.rec + (int64_t)dg * a.g.ncell + cc);
+    // thread t copies node t mod 128 of the plane (108 nodes) of every second direction
+    {
+        const int n = t % 128, prow = n / kPatchPitch, pcol = n - prow * kPatchPitch;
+        const int ni = x0 + pcol, nj = y0 + prow;
+        if (n < kPatchNodes && ni < nx && nj < (int)a.g.ny)
+        {
+            const double *src = a.Iin + ni + (int64_t)nj * nx;
+            for (int d = t / 128; d < nd; d += kPatchThreads / 128)
+                copy8_async(patch + d * kPatchPlane + n, src + (int64_t)d * nxy);
+        }
+    }
+    double2 *wrow = reinterpret_cast<double2 *>(cubes + 9 * kPatchCells);
+    int *brow = reinterpret_cast<int *>(wrow + 2 * a.ng);
+    for (int g = t; g < a.ng; g += kPatchThreads)
+    {
+        const IgRow *r0 = a.ig_rows + g, *r1 = a.ig_rows + (g + 1 == a.ng ? 0 : g + 1);
+        wrow[2 * g] = r0->w01;
+        wrow[2 * g + 1] = r0->w23;
+        brow[g] = 2 * r0->idx.x + (r1->idx.x != r0->idx.x);
+    }
+    if (active)
+        for (int n = dg; n < 9; n += kPatchDirs)
+            copy8_async(cubes + n * kPatchCells + cell, a.acube + ij + (int64_t)n * nxy);
+    asm volatile("cp.async.wait_all;\n" ::: "memory");
+    __syncthreads();
+    if (!active)
+        return;
+    unsigned far = 0; // this thread's directions (bit d / 4) that depart outside the 3x3 neighbourhood
+    static_assert(kPatchMaxDirs <= 32 * kPatchDirs, "one bit per direction of a thread");
+    for (int d = dg; d < nd; d += kPatchDirs)
+    {
+        const double4 rc = r;
+        if (streams && d + kPatchDirs < nd)
+            r = load_once(a.rec + (int64_t)(d + kPatchDirs) * a.g.ncell + cc);
+        unsigned cm = 0xFu;
+        double val = 0.0;
+        if (streams && !(rc.z < 0.0))
+        {
+            const int i0 = min(max((int)floor(rc.x), 0), nx - 2);
+            const int j0 = min(max((int)floor(rc.y), 0), (int)a.g.ny - 2);
+            if ((unsigned)(i0 - i + 1) <= 1u && (unsigned)(j0 - j + 1) <= 1u)
+            {
+                const int gz = (int)floor(rc.z);
+                int g0 = (unsigned)gz < (unsigned)a.ng ? gz : gz % a.ng;
+                g0 = g0 < 0 ? 0 : g0;
+                const int g1 = g0 + 1 == a.ng ? 0 : g0 + 1;
+                const double tt = rc.z - (double)g0, t1 = 1.0 - tt;
+                const int bs = brow[g0], b0 = bs >> 1;
+                const bool shift = bs & 1;
+                const double2 wa = wrow[2 * g0], wb = wrow[2 * g0 + 1], wc = wrow[2 * g1], wd = wrow[2 * g1 + 1];
+                const double *p[5];
+#pragma unroll
+                for (int k = 0; k < 5; k++)
+                {
+                    const int dk = b0 + k;
+                    p[k] = patch + ((dk >= nd ? dk - nd : dk) * kPatchPlane + (i0 - x0) + (j0 - y0) * kPatchPitch);
+                }
+                const double *cube00 = cubes + (3 * (j0 - j + 1) + (i0 - i + 1)) * kPatchCells + cell;
+                double Iq[4];
+#pragma unroll
+                for (int q = 0; q < 4; q++) // corners 00, 01, 10, 11
+                {
+                    const int off = (q >> 1) + (q & 1) * kPatchPitch;
+                    const double c0 = p[0][off], c1 = p[1][off], c2 = p[2][off], c3 = p[3][off], c4 = p[4][off];
+                    const double e0 = shift ? c1 : c0, e1 = shift ? c2 : c1, e2 = shift ? c3 : c2, e3 = shift ? c4 : c3;
+                    const double v0 = wa.x * c0 + wa.y * c1 + wb.x * c2 + wb.y * c3;
+                    const double v1 = wc.x * e0 + wc.y * e1 + wd.x * e2 + wd.y * e3;
+                    double v = v0 * t1 + v1 * tt;
+                    if (!(0.0 < v))
+                        cm &= ~(1u << q);
+                    v = (0.0 < v) ? v : 0.0;
+                    Iq[q] = cube00[((q >> 1) + 3 * (q & 1)) * kPatchCells] * v;
+                }
+                const double fx = rc.x - (double)i0, fy = rc.y - (double)j0;
+                const double f0 = Iq[0] * (1.0 - fx) + Iq[2] * fx;
+                const double f1 = Iq[1] * (1.0 - fx) + Iq[3] * fx;
+                val = rc.w * (f0 * (1.0 - fy) + f1 * fy);
+            }
+            else
+                far |= 1u << (d / kPatchDirs);
+        }
+        if (RECORD)
+            rec.clamp[(int64_t)d * a.g.ncell + cc] = (uint8_t)cm;
+        a.S[(int64_t)d * nxy + ij] = val;
+    }
+    // the rare far departures, from global memory
+    for (; far; far &= far - 1)
+    {
+        const int d = (__ffs((int)far) - 1) * kPatchDirs + dg;
+        unsigned cm;
+        a.S[(int64_t)d * nxy + ij] =
+            stream_value<true, int64_t>(a, d, load_once(a.rec + (int64_t)d * a.g.ncell + cc), i, j, ij, cm);
+        if (RECORD)
+            rec.clamp[(int64_t)d * a.g.ncell + cc] = (uint8_t)cm;
+    }
+}
+
 // Curved adaptive stream: a block takes 16 cells of one row for kPDirs
 // directions (16: 7% faster than 8, and 32 slower, at 400^2 x 64).  It first
 // stages the row's Fourier coefficients (5 nF x 16 doubles, at most 40 KB)
@@ -529,34 +562,83 @@ __global__ void __launch_bounds__(kAdaptiveBlock) k_stream_plain_curved_adaptive
     a.S[(int64_t)d * a.g.nxy + ij] = val;
 }
 
-// Moments and collide: one thread per cell sums the moments of its streamed
-// values in direction order (ComputeMomentsIF's order, as the fused step
-// does) and finishes the cell; the collided intensities go to Iout.  With
-// COLUMN (when the block's values fit in 48 KB of shared memory) each thread
-// keeps its cell's streamed values in its own column of shared memory for
-// the lambda iteration's passes, instead of re-reading them from L2.
+// The lambda iteration's exit test (src/Radiation.cpp:714-721): whether
+// sqrt(sum ((p - m) / m)^2) over the six moments is above 1e-4.  The sum is
+// first taken in FP32 (within 1e-5 of itself while every moment is in FP32's
+// range); only where that is within 0.1% of the limit, or not in range, are
+// the six quotients and the root taken as the reference does.
+__device__ __forceinline__ bool still_changing(const double (&p)[6], const double (&m)[6])
+{
+    float s = 0.f, lo = 1e30f, hi = 0.f;
+#pragma unroll
+    for (int q = 0; q < 6; q++)
+    {
+        const float d = (float)(p[q] - m[q]), f = (float)m[q], x = __fdividef(d, f);
+        s += x * x;
+        lo = fminf(lo, fabsf(f));
+        hi = fmaxf(hi, fabsf(f));
+        // a difference below FP32's normal range counts as out of range, zero does not
+        if (d != 0.f && fabsf(d) < 1e-30f)
+            lo = 0.f;
+    }
+    if (lo > 1e-30f && hi < 1e30f && (s > 1.001e-8f || s < 0.999e-8f) && s < 1e30f)
+        return s > 1e-8f;
+    double e = 0.0, ee[6];
+#pragma unroll
+    for (int q = 0; q < 6; q++)
+        ee[q] = (p[q] - m[q]) / m[q];
+    e = ee[0] * ee[0] + ee[1] * ee[1] + ee[2] * ee[2] + ee[3] * ee[3] + ee[4] * ee[4] + ee[5] * ee[5];
+    return fabs(sqrt(e)) > 1e-4;
+}
+
+// Moments and collide of the streamed values: one thread per cell sums the
+// moments in direction order (ComputeMomentsIF's order), runs the lambda
+// iteration (src/Radiation.cpp:641-736) and writes the collided intensities.
+// The order of a moment's sum is the reference's, so a cell's passes over the
+// directions are serial and the kernel is bound by issuing them: with COLUMN
+// (up to kColumnMaxDirs directions) each cell's streamed values wait in a
+// column of shared memory, and the passes of a fluid at rest without anisotropic
+// scattering are stripped to the 17 FP64 operations per direction that the
+// roundings need.  (Two lanes per cell, sharing the quotients and the six
+// sums, doubled the warps but took a third more operations: 183 us against
+// 134 at 400^2 x 64.)
 constexpr int kColumnTileY = 4; // 16 x 4 cells per block with COLUMN
+constexpr int kColumnMaxDirs = 90; // the column and the tables within 48 KB
+#ifndef GRLBM_COLLIDE_MIN_BLOCKS
+#define GRLBM_COLLIDE_MIN_BLOCKS 6
+#endif
+#ifndef GRLBM_COLLIDE_UNROLL
+#define GRLBM_COLLIDE_UNROLL 8
+#endif
+constexpr int kCollideUnroll = GRLBM_COLLIDE_UNROLL;
+constexpr size_t collide_smem(int nd, bool column)
+{
+    return (size_t)nd * (4 + (column ? kSplitTileX * kColumnTileY : 0)) * sizeof(double);
+}
 template <bool RECORD, bool ADAPTIVE, bool COLUMN>
-__global__ void __launch_bounds__(kStepBlock) k_collide_plain(PlainStepArgs a, StepRecord rec)
+__global__ void __launch_bounds__(COLUMN ? kSplitTileX *kColumnTileY : kStepBlock, COLUMN ? GRLBM_COLLIDE_MIN_BLOCKS : 4)
+    k_collide_plain(const __grid_constant__ PlainStepArgs a, const __grid_constant__ StepRecord rec)
 {
     constexpr int TY = COLUMN ? kColumnTileY : kSplitTileY, NT = kSplitTileX * TY;
+    extern __shared__ __align__(16) double dyn[]; // {n1, n2, w, 0} per direction, then the values [d][cell]
     const int t = threadIdx.x;
     const int ti = 1 + (int)blockIdx.x * kSplitTileX + t % kSplitTileX;
     const int tj = (int)a.g.jlo + (int)blockIdx.y * TY + t / kSplitTileX;
     const bool active = ti <= a.g.nx_ && tj < a.g.jhi;
     const int64_t i = active ? ti : 1, j = active ? tj : 1;
-    const int64_t cc = (i - 1) + (j - 1) * a.g.nx_;
     const int64_t ij = i + j * a.g.nx;
     const int64_t nxy = a.g.nxy;
-    const bool collides = active && !(a.flags[ij] & 1);
-    // the stencil's weights and directions, read by every cell of the block
-    extern __shared__ double dyn[];
-    double *sw = dyn, *sn1 = dyn + a.nd, *sn2 = dyn + 2 * a.nd;
+    const int nd = a.nd;
+    const double *S = a.S + ij;
+    double2 *dir = reinterpret_cast<double2 *>(dyn);
+    double *col = dyn + 4 * nd + t;
     const double *dn1 = ADAPTIVE ? a.cx : a.n1, *dn2 = ADAPTIVE ? a.cy : a.n2;
-    for (int d = t; d < a.nd; d += NT)
-        sw[d] = a.w[d], sn1[d] = dn1[d], sn2[d] = dn2[d];
-    __syncthreads();
-    const double *tw = sw, *tn1 = sn1, *tn2 = sn2;
+    for (int d = t; d < nd; d += NT)
+    {
+        dir[2 * d] = make_double2(dn1[d], dn2[d]);
+        dir[2 * d + 1] = make_double2(a.w[d], 0.0);
+    }
+    const bool collides = active && !(a.flags[ij] & 1);
     // the cell's rotation (adaptive streaming)
     double rot_s = 0.0, rot_c = 1.0;
     if (ADAPTIVE)
@@ -565,26 +647,178 @@ __global__ void __launch_bounds__(kStepBlock) k_collide_plain(PlainStepArgs a, S
         rot_s = rn.x;
         rot_c = rn.y;
     }
-    const double *S = a.S + ij;
-    double *col = dyn + 3 * a.nd + t; // COLUMN: this cell's values, stride NT
+    __syncthreads();
+    auto streamed = [&](int d) { return COLUMN ? col[d * NT] : S[(int64_t)d * nxy]; };
+    // direction d of the cell's stencil
+    auto direction = [&](int d) {
+        const double2 n = dir[2 * d];
+        return ADAPTIVE ? make_double2(n.x * rot_c - n.y * rot_s, n.x * rot_s + n.y * rot_c) : n;
+    };
     Moments m;
     m.zero();
+    // the streamed values' high words: the range of the quotients' shortcut
+    unsigned least = 0x7fffffffu, most = 0u;
     if (active)
     {
-#pragma unroll kCollideUnroll
-        for (int d = 0; d < a.nd; d++)
+#pragma unroll 8
+        for (int d = 0; d < nd; d++)
         {
             const double v = S[(int64_t)d * nxy];
             if (COLUMN)
                 col[d * NT] = v;
-            m.add(tw[d], v, GRLBM_N1(d), GRLBM_N2(d));
+            const double2 n = direction(d);
+            const unsigned hi = (unsigned)__double2hiint(v);
+            most = max(most, hi);
+            least = min(least, (hi | (unsigned)__double2loint(v)) == 0u ? 0x7fffffffu : hi);
+            m.add(dir[2 * d + 1].x, v, n.x, n.y);
         }
     }
-    finish_cell<RECORD, ADAPTIVE>(a, rec, active, collides, ij, cc, m, COLUMN ? col : S, COLUMN ? NT : nxy,
-                                  a.Iout + ij, rot_s, rot_c, tw, tn1, tn2);
+    const int64_t cc = (i - 1) + (j - 1) * a.g.nx_;
+    if (RECORD && active)
+        rec.e0[cc] = m.E;
+    int cycles = 0;
+    if (collides)
+    {
+        const double u1 = a.u1[ij], u2 = a.u2[ij], lor = a.lor[ij], adt = a.adt[ij];
+        const double eta = a.eta[ij], k0 = a.k0[ij], k3 = a.k3[ij], kak0 = a.ka[ij] + a.k0[ij];
+        // A fluid at rest has u = 0 and lorentz = 1, so in collide_value
+        // A = 1, n_ff = n and AA = 1 exactly: the update reduces to
+        // (I + adt (eta + (k0 fE + k3 (n1 fFx + n2 fFy)))) / (1 + adt kak0)
+        // with the same roundings.
+        const bool rest = u1 == 0.0 && u2 == 0.0 && lor == 1.0;
+        const double den = 1.0 + adt * kak0;
+        const bool fast_div = rest && den >= 1.0 && den < 0x1p+100;
+        const double rden = __drcp_rn(den);
+        double fE = 0, fFx = 0, fFy = 0;
+        // Without anisotropic scattering (3 kappa1 = 0) the source
+        // adt (eta + (k0 fE + 0 (n . fF))) of a fluid at rest is the same
+        // number for every direction as long as fF is finite: `src`, worked
+        // out once per cycle.  `plain`: every S + src is also zero or in the
+        // range of div_rn's shortcut (no negative terms, none tiny or huge).
+        bool iso = false, plain = false;
+        double src = 0.0;
+        auto quotient_plain = [&](double num) {
+            double q = __dmul_rn(num, rden);
+            q = __fma_rn(__fma_rn(-q, den, num), rden, q);
+            return __fma_rn(__fma_rn(-q, den, num), rden, q);
+        };
+        auto value = [&](int d, double2 n) {
+            const double num = streamed(d) + (iso ? src : adt * (eta + (k0 * fE + k3 * (n.x * fFx + n.y * fFy))));
+            return fast_div ? div_rn(num, den, rden) : num / den;
+        };
+        bool more = true;
+        do
+        {
+            cycles++;
+            const double p[6] = {m.E, m.Fx, m.Fy, m.Pxx, m.Pxy, m.Pyy};
+            const bool was_iso = iso;
+            if (rest && fabs(p[0]) < 1e300 && fabs(p[1]) < 1e300 && fabs(p[2]) < 1e300 && fabs(p[3]) < 1e300 &&
+                fabs(p[4]) < 1e300 && fabs(p[5]) < 1e300)
+            {
+                // the transform below with u = 0, lorentz = 1 and finite moments
+                fE = p[0];
+                fFx = p[1];
+                fFy = p[2];
+                iso = k3 == 0.0;
+            }
+            else
+            {
+                // fluid-frame moments of the previous iterate (src/Radiation.cpp:672-678)
+                const double uF = u1 * p[1] + u2 * p[2];
+                const double uxP = u1 * p[3] + u2 * p[4];
+                const double uyP = u1 * p[4] + u2 * p[5];
+                const double uuP = u1 * uxP + u2 * uyP;
+                fE = lor * lor * (p[0] - 2.0 * uF + uuP);
+                fFx = lor * lor * (p[1] - lor * p[0] * u1 - uxP + u1 * lor / (1.0 + lor) * ((2.0 * lor + 1.0) * uF - lor * uuP));
+                fFy = lor * lor * (p[2] - lor * p[0] * u2 - uyP + u2 * lor / (1.0 + lor) * ((2.0 * lor + 1.0) * uF - lor * uuP));
+                iso = false;
+            }
+            if (iso)
+            {
+                const double before = src;
+                src = adt * (eta + k0 * fE);
+                // The same source as in the cycle before (always so without
+                // scattering), or in the first cycle nothing to absorb,
+                // scatter or emit: the cycle would find the moments that m
+                // already holds, and relative changes of 0 (or 0 / 0), which
+                // end the iteration.
+                if (cycles > 1 ? was_iso && src == before : src == 0.0 && den == 1.0)
+                    break;
+                const unsigned hs = (unsigned)__double2hiint(src);
+                plain = fast_div && most < 0x70000000u && least > 0x0b000000u &&
+                        (src == 0.0 || (hs > 0x0b000000u && hs < 0x70000000u));
+            }
+            m.zero();
+            if (iso && plain)
+            {
+#pragma unroll kCollideUnroll
+                for (int d = 0; d < nd; d++)
+                {
+                    const double2 n = direction(d);
+                    m.add(dir[2 * d + 1].x, quotient_plain(streamed(d) + src), n.x, n.y);
+                }
+            }
+            else if (rest)
+                for (int d = 0; d < nd; d++)
+                {
+                    const double2 n = direction(d);
+                    m.add(dir[2 * d + 1].x, value(d, n), n.x, n.y);
+                }
+            else
+                for (int d = 0; d < nd; d++)
+                {
+                    const double2 n = direction(d);
+                    const double v =
+                        collide_value(streamed(d), n.x, n.y, u1, u2, lor, adt, eta, k0, k3, kak0, fE, fFx, fFy);
+                    m.add(dir[2 * d + 1].x, v, n.x, n.y);
+                }
+            const double q[6] = {m.E, m.Fx, m.Fy, m.Pxx, m.Pxy, m.Pyy};
+            more = still_changing(p, q);
+        } while (more && cycles < 100);
+        // the last iterate, recomputed from the same operands
+        double *out = a.Iout + ij;
+        if (iso && plain)
+        {
+#pragma unroll kCollideUnroll
+            for (int d = 0; d < nd; d++)
+                out[(int64_t)d * nxy] = quotient_plain(streamed(d) + src);
+        }
+        else if (rest)
+            for (int d = 0; d < nd; d++)
+                out[(int64_t)d * nxy] = value(d, direction(d));
+        else
+            for (int d = 0; d < nd; d++)
+            {
+                const double2 n = direction(d);
+                out[(int64_t)d * nxy] =
+                    collide_value(streamed(d), n.x, n.y, u1, u2, lor, adt, eta, k0, k3, kak0, fE, fFx, fFy);
+            }
+    }
+    if (RECORD && active)
+        rec.cycles[cc] = cycles;
+    if (active)
+    {
+        a.mom[ij] = m.E;
+        a.mom[ij + nxy] = m.Fx;
+        a.mom[ij + 2 * nxy] = m.Fy;
+        a.mom[ij + 3 * nxy] = m.Pxx;
+        a.mom[ij + 4 * nxy] = m.Pxy;
+        a.mom[ij + 5 * nxy] = m.Pyy;
+    }
+    // lambda-iteration statistics: warp sums and maxima, one atomic per warp
+    unsigned sum = (unsigned)cycles, mx = (unsigned)cycles;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1)
+    {
+        sum += __shfl_xor_sync(0xffffffffu, sum, o);
+        mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+    }
+    if ((t & 31) == 0 && sum)
+    {
+        atomicAdd(a.iter_sum, (unsigned long long)sum);
+        atomicMax(a.iter_max, mx);
+    }
 }
-#undef GRLBM_N1
-#undef GRLBM_N2
 
 // UpdateRotationMatrizes (src/Radiation.cpp:361-378): for the interior cells
 // of the slab, the angle of the flux averaged over the 3x3 neighbourhood
@@ -871,8 +1105,18 @@ inline unsigned nblk(int64_t n, int b) { return (unsigned)((n + b - 1) / b); }
 
 cudaError_t prepare_step_plain(int smem_bytes)
 {
-    (void)smem_bytes; // the plain step uses no dynamic shared memory
-    return cudaSuccess;
+    (void)smem_bytes;
+    const int patch = (int)patch_smem(kPatchMaxDirs);
+    cudaError_t e = cudaSuccess;
+    auto limit = [&](const void *f, int bytes) {
+        if (e == cudaSuccess)
+            e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    };
+    limit((const void *)k_stream_plain_patch<false, 4>, patch);
+    limit((const void *)k_stream_plain_patch<true, 4>, patch);
+    limit((const void *)k_stream_plain_patch<false, 6>, patch);
+    limit((const void *)k_stream_plain_patch<true, 6>, patch);
+    return e;
 }
 void launch_step_plain(const PlainStepArgs &a, bool curved, cudaStream_t s, const StepRecord *record)
 {
@@ -883,7 +1127,7 @@ void launch_step_plain(const PlainStepArgs &a, bool curved, cudaStream_t s, cons
     const StepRecord none{};
     const StepRecord &rec = record && !adaptive ? *record : none;
     const unsigned tx = nblk(a.g.nx_, kSplitTileX), ty = nblk(a.g.jhi - a.g.jlo, kSplitTileY);
-    const dim3 sgrid(tx, ty, (unsigned)a.nd), sgrid_df((unsigned)a.nd, tx, ty), cgrid(tx, ty);
+    const dim3 sgrid(tx, ty, (unsigned)a.nd), sgrid_df((unsigned)a.nd, tx, ty);
     if (adaptive) // UpdateRotationMatrizes from the previous moments, before the stream
     {
         k_rotation_update<double><<<nblk(cells, 128), 128, 0, s>>>(a.g, a.mom, a.ang_old, const_cast<double *>(a.ang_new));
@@ -897,6 +1141,17 @@ void launch_step_plain(const PlainStepArgs &a, bool curved, cudaStream_t s, cons
                                          (size_t)5 * a.nf * kSplitTileX * sizeof(double), s>>>(a);
     else if (adaptive)
         k_stream_plain<false, false, true><<<ga, kStepBlock, 0, s>>>(a, rec);
+    else if (curved && a.nd <= kPatchMaxDirs && !a.wide)
+    {
+        const dim3 pgrid(nblk(a.g.nx_, kPatchX), nblk(a.g.jhi - a.g.jlo, kPatchY));
+        const size_t sm = patch_smem(a.nd);
+        if (a.nd <= kPatchFewDirs)
+            record ? k_stream_plain_patch<true, 4><<<pgrid, 4 * kPatchCells, sm, s>>>(a, rec)
+                   : k_stream_plain_patch<false, 4><<<pgrid, 4 * kPatchCells, sm, s>>>(a, rec);
+        else
+            record ? k_stream_plain_patch<true, 6><<<pgrid, 6 * kPatchCells, sm, s>>>(a, rec)
+                   : k_stream_plain_patch<false, 6><<<pgrid, 6 * kPatchCells, sm, s>>>(a, rec);
+    }
     else if (curved && a.wide) // 64-bit state offsets
         record ? k_stream_plain<true, true, false, true><<<gf, kStepBlock, 0, s>>>(a, rec)
                : k_stream_plain<true, false, false, true><<<gf, kStepBlock, 0, s>>>(a, rec);
@@ -907,25 +1162,20 @@ void launch_step_plain(const PlainStepArgs &a, bool curved, cudaStream_t s, cons
         record ? k_stream_plain<false, true, false><<<gf, kStepBlock, 0, s>>>(a, rec)
                : k_stream_plain<false, false, false><<<gf, kStepBlock, 0, s>>>(a, rec);
     // moments and collide: with each cell's values in shared memory when they fit
-    const size_t tables = 3 * (size_t)a.nd * sizeof(double);
-    const size_t column = tables + (size_t)a.nd * kSplitTileX * kColumnTileY * sizeof(double);
-    if (column <= 48 * 1024)
-    {
-        const dim3 kgrid(tx, nblk(a.g.jhi - a.g.jlo, kColumnTileY));
-        const unsigned nt = kSplitTileX * kColumnTileY;
-        if (adaptive)
-            k_collide_plain<false, true, true><<<kgrid, nt, column, s>>>(a, rec);
-        else if (record)
-            k_collide_plain<true, false, true><<<kgrid, nt, column, s>>>(a, rec);
-        else
-            k_collide_plain<false, false, true><<<kgrid, nt, column, s>>>(a, rec);
-    }
-    else if (adaptive)
-        k_collide_plain<false, true, false><<<cgrid, kStepBlock, tables, s>>>(a, rec);
+    const bool column = a.nd <= kColumnMaxDirs;
+    const dim3 kgrid(tx, column ? nblk(a.g.jhi - a.g.jlo, kColumnTileY) : ty);
+    const unsigned kthreads = column ? kSplitTileX * kColumnTileY : kStepBlock;
+    const size_t ksmem = collide_smem(a.nd, column);
+    static_assert(collide_smem(kColumnMaxDirs, true) <= 48 * 1024, "within the default limit");
+    if (adaptive)
+        column ? k_collide_plain<false, true, true><<<kgrid, kthreads, ksmem, s>>>(a, rec)
+               : k_collide_plain<false, true, false><<<kgrid, kthreads, ksmem, s>>>(a, rec);
     else if (record)
-        k_collide_plain<true, false, false><<<cgrid, kStepBlock, tables, s>>>(a, rec);
+        column ? k_collide_plain<true, false, true><<<kgrid, kthreads, ksmem, s>>>(a, rec)
+               : k_collide_plain<true, false, false><<<kgrid, kthreads, ksmem, s>>>(a, rec);
     else
-        k_collide_plain<false, false, false><<<cgrid, kStepBlock, tables, s>>>(a, rec);
+        column ? k_collide_plain<false, false, true><<<kgrid, kthreads, ksmem, s>>>(a, rec)
+               : k_collide_plain<false, false, false><<<kgrid, kthreads, ksmem, s>>>(a, rec);
     if (adaptive) // the halo moments, recomputed by the reference from unwritten (zero) intensities
         k_zero_halo_moments<double><<<nblk(a.g.nxy, 256), 256, 0, s>>>(a.g, a.mom);
 }

@@ -529,7 +529,7 @@ __global__ void k_alpha_cube(GridDev g, const double *alpha, double *acube)
         for (int di = -1; di <= 1; di++)
         {
             const double r = al / alpha[ij + di + dj * g.nx];
-            acube[ij * 9 + 3 * (dj + 1) + (di + 1)] = r * (r * r);
+            acube[ij + (3 * (dj + 1) + (di + 1)) * g.nxy] = r * (r * r);
         }
 }
 
