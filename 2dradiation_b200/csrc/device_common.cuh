@@ -1,8 +1,9 @@
 // Types and launch entry points shared by the kernel translation units.
 //
 // Translation units and their floating-point contracts:
-//   kernels_tables.cu    geodesic backtrace, Fourier projection, departure
-//                        records, alpha-ratio cubes -- FP64, built with
+//   kernels_geodesic.cu  geodesic backtrace and Fourier projection -- FP64,
+//                        contracted FMAs in the backtrace
+//   kernels_tables.cu    departure records, alpha-ratio cubes -- FP64, built with
 //                        -fmad=false (every product rounded once, as on the
 //                        reference's CPU)
 //   kernels_plain.cu     the plain FP64 step (stream + moments + collide),
@@ -146,21 +147,12 @@ struct GeodesicArgs
     int nf;
     double tol;
     int max_trials;
-    double *data; // out: [5][cn][nf]: 1/s, x, y, vIF_x, vIF_y of the built cells
+    const double *ss_w;  // nf: the streaming stencil's weights
+    const double *basis; // [f][k] = Basis(k, phi_f)
+    double *coef;        // out: [5][nxy][nf], the built cells' coefficients
     unsigned long long *trials_total;
     int *nonconverged;
-    int64_t c0, cn; // the interior cells built: [c0, c0 + cn)
-};
-
-struct ProjectArgs
-{
-    GridDev g;
-    int nf;
-    const double *data;  // [5][ncell][nf]
-    const double *ss_w;  // nf
-    const double *basis; // [f][k] = Basis(k, phi_f)
-    double *coef;        // [5][nxy][nf]
-    int64_t c0, cn;      // the interior cells built (data holds them): [c0, c0 + cn)
+    int64_t c0, cn; // the interior cells built, whole rows: [c0, c0 + cn)
 };
 
 // Directions per chunk of the adaptive precision-form kernels' moment loops.
@@ -451,7 +443,6 @@ void set_global_error(const char *msg);
 
 // ---- launchers (defined in the kernel translation units) ----
 void launch_geodesic(const GeodesicArgs &a, cudaStream_t s);
-void launch_project(const ProjectArgs &a, cudaStream_t s);
 void launch_departure(const DepartureArgs &a, cudaStream_t s);
 void launch_alpha_cube(const GridDev &g, const double *alpha, double *acube, cudaStream_t s);
 

@@ -1490,8 +1490,6 @@ int grlbm_update_fourier_coefficients(grlbm_ctx *ctx, double rk_tol, int32_t max
     const int64_t c0 = (ctx->gd.jlo - 1) * ctx->gd.nx_, cn = (ctx->gd.jhi - ctx->gd.jlo) * ctx->gd.nx_;
     unsigned long long *cnt = ctx->counters.as<unsigned long long>();
     CU(cudaMemsetAsync(cnt + 2, 0, 2 * sizeof(unsigned long long), ctx->stream));
-    void *data = nullptr;
-    CU(cudaMallocAsync(&data, (size_t)5 * cn * nf * sizeof(double), ctx->stream));
     cudaEvent_t e0, e1;
     cudaEventCreate(&e0);
     cudaEventCreate(&e1);
@@ -1505,27 +1503,18 @@ int grlbm_update_fourier_coefficients(grlbm_ctx *ctx, double rk_tol, int32_t max
     ga.nf = nf;
     ga.tol = rk_tol;
     ga.max_trials = max_substeps > 0 ? max_substeps : 1000000;
-    ga.data = static_cast<double *>(data);
+    ga.ss_w = ctx->ss_w.as<double>();
+    ga.basis = ctx->proj_basis.as<double>();
+    ga.coef = ctx->coef.as<double>();
     ga.trials_total = cnt + 2;
     ga.nonconverged = reinterpret_cast<int *>(cnt + 3);
     ga.c0 = c0;
     ga.cn = cn;
     launch_geodesic(ga, ctx->stream);
 
-    ProjectArgs pa{};
-    pa.g = ctx->gd;
-    pa.nf = nf;
-    pa.data = ga.data;
-    pa.ss_w = ctx->ss_w.as<double>();
-    pa.basis = ctx->proj_basis.as<double>();
-    pa.coef = ctx->coef.as<double>();
-    pa.c0 = c0;
-    pa.cn = cn;
-    launch_project(pa, ctx->stream);
     int rc = build_records(ctx);
     cudaEventRecord(e1, ctx->stream);
     cudaError_t le = cudaGetLastError();
-    cudaFreeAsync(data, ctx->stream);
     cudaError_t se = cudaStreamSynchronize(ctx->stream);
     float ms = 0;
     cudaEventElapsedTime(&ms, e0, e1);
