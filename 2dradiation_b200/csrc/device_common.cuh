@@ -404,6 +404,21 @@ struct Step64Args
     CUtensorMap in_map;      // Iin as a 4D tensor, one box per tile patch (encode_state_map64)
 };
 
+// The fixed streaming types' step with one patch per block (step_block.cuh):
+// a block's tile is kBlockStepWarps rows of 8 or 4 cells, one per warp.
+constexpr int kBlockStepWarps = 8;
+struct BlockStep
+{
+    int run;                 // cells of a row a warp takes: a tile is `run` x kBlockStepWarps cells
+    int tiles_x, tiles_y;    // tiles over the slab rows
+    int ss;                  // row stride of the streamed values
+    int q, nd4;              // row types; directions rounded up to 4
+    int parts;               // lanes that share a run's cells of one direction (flat streaming)
+    int off_wmom, off_rows, off_mom, off_dir, off_flat, off_map, off_patch, off_s; // shared memory, bytes
+    int smem;                // a block's dynamic shared memory (0: the step runs the warp-per-tile kernel)
+    CUtensorMap map;         // the state read, one box per tile patch
+};
+
 // Direction tables of the fast FP64 step (device memory, copied into each
 // block's shared memory): the angular rows and moment coefficients of
 // DirTable in FP64, and the flat departures' products c dt.
@@ -484,6 +499,11 @@ void launch_step32(const Step32Args &a, const DirTable &dt, bool curved, int P, 
 void launch_step_batch32(const Batch32Item *items, const int *first_tile, int n_items, int total_tiles, int flip,
                          unsigned *counters, int P, int blocks, size_t smem, int warp_stride, int s_offset,
                          int item_bytes, cudaStream_t s);
+// The one-patch-per-block step (step_block.cuh): shared memory of a tile
+// (b.run set), its resident blocks per SM, and the launch.
+void block_layout32(BlockStep &b, int nd, int dp, int q, bool curved);
+cudaError_t block_occupancy32(bool curved, int run, int smem, int *blocks);
+void launch_step_block32(const Step32Args &a, const BlockStep &b, const DirTable *dt, bool curved, cudaStream_t s);
 // The TMA map the step stages a cell-major state of nx x ny nodes through,
 // for tiles of tx x ty cells.
 cudaError_t encode_state_map32(CUtensorMap *map, const float *state, int64_t nx, int64_t ny, int dp, int tx, int ty);
@@ -497,6 +517,9 @@ int step64_warp_stride(int tx, int ty, int dp, int nd);
 size_t step64_smem(int tx, int ty, int dp, int nd, int q);
 cudaError_t prepare_step64();
 cudaError_t step64_occupancy(int P, bool curved, size_t smem, int *blocks);
+void block_layout64(BlockStep &b, int nd, int dp, int q, bool curved);
+cudaError_t block_occupancy64(bool curved, int run, int smem, int *blocks);
+void launch_step_block64(const Step64Args &a, const BlockStep &b, const DirTable64 *dt, bool curved, cudaStream_t s);
 void launch_step64(const Step64Args &a, const DirTable64 *dt, bool curved, int P, int blocks, cudaStream_t s);
 cudaError_t encode_state_map64(CUtensorMap *map, const double *state, int64_t nx, int64_t ny, int dp, int tx, int ty);
 

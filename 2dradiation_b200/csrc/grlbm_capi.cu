@@ -62,6 +62,7 @@ struct grlbm_ctx
     // persistent grid, and the TMA maps of the state buffers for that tile
     int tile_x = 4, tile_y = 4, passes = 1, step_blocks = 1;
     CUtensorMap in_map[2];
+    BlockStep blk[2] = {}; // blk[k]: the one-patch-per-block step that reads buffer k (smem 0: not used)
     unsigned *fault = nullptr; // mapped host word: a precision step's staging wait timed out
     int64_t ncell = 0;
     int ng = 0;
@@ -81,6 +82,7 @@ struct grlbm_ctx
     DevBuf streamed; // plain form: the streamed values of a step
     DevBuf coef_k;   // adaptive streaming: the coefficients as [5][nf][nxy]
     DirTable dirs{}; // precision-form direction tables (kernel parameter)
+    DevBuf dirs32t;  // the precision form's direction tables (a DirTable in device memory)
     DevBuf dirs64t;  // the fast FP64 form's direction tables (a DirTable64 in device memory)
     DevBuf cu1, cu2, clor, cadt, ceta, ck0, ck3, cka, mom, rkf, lfp;
     DevBuf coef, ss_cx, ss_cy, ss_w, proj_basis, eval_basis, stage;
@@ -424,6 +426,7 @@ int set_step32_tile(grlbm_ctx *ctx, int tx, int ty)
     ctx->tile_x = tx;
     ctx->tile_y = ty;
     ctx->step_blocks = per_sm * sms;
+    ctx->blk[0].smem = ctx->blk[1].smem = 0; // a tile asked for: the warp-per-tile kernel
     invalidate_graphs(ctx);
     return GRLBM_OK;
 }
@@ -462,6 +465,61 @@ int adaptive_departure_rows(grlbm_ctx *ctx, int32_t *rows)
     }
     *rows = (int32_t)std::floor(far + 1e-3) + 1;
     return GRLBM_OK;
+}
+
+// Sets up the one-patch-per-block step, the default where its patch fits an
+// SM (the warp-per-tile kernel runs where a tile shape is asked for, in the
+// persistent batch launch, and for the direction counts whose patch does not
+// fit).  A warp takes 8 cells of a row, or 4 where 8 would leave the GPU
+// idle: at most one tile for every second SM (64^2 x 64 directions, fast FP64:
+// 8.2 against 9.0 us), or one block an SM where 4 give two (100^2 x 200:
+// FP32 29.6 against 38.2 us, fast FP64 53 against 92 us; 200^2 x 96 in fast
+// FP64: 73 against 80 us).  Elsewhere 8: a run's fixed work is halved (400^2 x
+// 64: FP32 82 against 105 us, fast FP64 154 against 191 us).
+int set_block_step(grlbm_ctx *ctx)
+{
+    const bool curved = ctx->run.streaming_type == GRLBM_CURVED_FIXED;
+    const int dp = (int)ctx->sl.sp;
+    int sms = 0;
+    CU(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device));
+    BlockStep b[2] = {}; // runs of 8, of 4
+    int per_sm[2] = {0, 0};
+    for (int k = 0; k < 2; k++)
+    {
+        b[k].run = k ? 4 : 8;
+        if (ctx->fast64)
+            block_layout64(b[k], ctx->st.n, dp, ctx->dirs.q, curved);
+        else
+            block_layout32(b[k], ctx->st.n, dp, ctx->dirs.q, curved);
+        if (b[k].smem <= kStep32MaxSmem)
+            CU(ctx->fast64 ? block_occupancy64(curved, b[k].run, b[k].smem, &per_sm[k])
+                           : block_occupancy32(curved, b[k].run, b[k].smem, &per_sm[k]));
+    }
+    const int64_t tiles = ((ctx->gd.nx_ + 7) / 8) * ((ctx->gd.jhi - ctx->gd.jlo + kBlockStepWarps - 1) / kBlockStepWarps);
+    const int pick = per_sm[0] < 1 || (per_sm[0] == 1 && per_sm[1] > 1) || 2 * tiles <= sms ? 1 : 0;
+    if (per_sm[pick] < 1)
+        return GRLBM_OK;
+    for (int k = 0; k < 2; k++)
+    {
+        ctx->blk[k] = b[pick];
+        const cudaError_t e = ctx->fast64 ? encode_state_map64(&ctx->blk[k].map, ctx->I[k].as<double>(), ctx->geo.nx,
+                                                               ctx->geo.ny, dp, b[pick].run, kBlockStepWarps)
+                                          : encode_state_map32(&ctx->blk[k].map, ctx->I[k].as<float>(), ctx->geo.nx,
+                                                               ctx->geo.ny, dp, b[pick].run, kBlockStepWarps);
+        if (e != cudaSuccess)
+            return fail(ctx, GRLBM_ERR_CUDA, "TMA map of the state: %s", cudaGetErrorString(e));
+    }
+    return GRLBM_OK;
+}
+
+// The block step's tiles over the rows of the context's band.
+BlockStep block_step(const grlbm_ctx *ctx, int from)
+{
+    BlockStep b = ctx->blk[from];
+    const int64_t rows = ctx->gd.jhi - ctx->gd.jlo;
+    b.tiles_x = (int)((ctx->gd.nx_ + b.run - 1) / b.run);
+    b.tiles_y = rows <= 0 ? 0 : (int)((rows + kBlockStepWarps - 1) / kBlockStepWarps);
+    return b;
 }
 
 // The default tile: the candidate with the most cells times resident blocks
@@ -515,7 +573,8 @@ int default_step32_tile(grlbm_ctx *ctx)
             if (max_cells < kStep32UnitCells)
                 continue;
         }
-        return set_step32_tile(ctx, cand[best][0], cand[best][1]);
+        const int rc = set_step32_tile(ctx, cand[best][0], cand[best][1]);
+        return rc ? rc : set_block_step(ctx);
     }
     return GRLBM_OK;
 }
@@ -596,15 +655,22 @@ int enqueue_step(grlbm_ctx *ctx, int from, bool sources = true, int blocks = 0)
         if (sources && ctx->run.keep_source_nodes_active && ctx->nsrc > 0)
             launch_sources64L(ctx->I[from].as<double>(), ctx->sl, ctx->st.n, ctx->src_nodes.as<int64_t>(),
                               ctx->src_vals.as<double>(), ctx->nsrc, ctx->stream);
-        launch_step64(step64_args(ctx, from), ctx->dirs64t.as<DirTable64>(), curved, ctx->passes, blocks,
-                      ctx->stream);
+        if (ctx->blk[from].smem)
+            launch_step_block64(step64_args(ctx, from), block_step(ctx, from), ctx->dirs64t.as<DirTable64>(), curved,
+                                ctx->stream);
+        else
+            launch_step64(step64_args(ctx, from), ctx->dirs64t.as<DirTable64>(), curved, ctx->passes, blocks,
+                          ctx->stream);
     }
     else if (ctx->fp32)
     {
         if (sources && ctx->run.keep_source_nodes_active && ctx->nsrc > 0)
             launch_sources32(ctx->I[from].as<float>(), ctx->sl, ctx->st.n, ctx->src_nodes.as<int64_t>(),
                              ctx->src_vals.as<float>(), ctx->nsrc, ctx->stream);
-        if (!is_adaptive(ctx))
+        if (ctx->blk[from].smem)
+            launch_step_block32(step32_args(ctx, from), block_step(ctx, from), ctx->dirs32t.as<DirTable>(), curved,
+                                ctx->stream);
+        else if (!is_adaptive(ctx))
             launch_step32(step32_args(ctx, from), ctx->dirs, curved, ctx->passes, blocks, ctx->stream);
         else
         {
@@ -1079,6 +1145,11 @@ int grlbm_create(const grlbm_grid_desc *grid, const grlbm_metric_desc *metric, c
         }
         for (int q = 0; q < 18; q++)
             dt.wmom[q] = (float)wm[q];
+        if (is_fixed32(ctx))
+        {
+            const std::vector<DirTable> one(1, dt);
+            TRY(upload(ctx, ctx->dirs32t, one));
+        }
         if (t64)
         {
             t64->q = q;
@@ -2753,6 +2824,7 @@ int grlbm_batch_autotune(grlbm_batch *b, int32_t trial_steps, int32_t *blocks_pe
         {
             grlbm_ctx *c0 = cls.second[0];
             int bx = c0->tile_x, by = c0->tile_y;
+            bool block = c0->blk[0].smem != 0; // the fastest so far is the block step
             double wc = 0.0;
             for (grlbm_ctx *c : cls.second)
                 wc += batch_cost(c);
@@ -2760,7 +2832,7 @@ int grlbm_batch_autotune(grlbm_batch *b, int32_t trial_steps, int32_t *blocks_pe
                 continue;
             for (const auto &t : cand)
             {
-                if (t[0] == bx && t[1] == by)
+                if (!block && t[0] == bx && t[1] == by)
                     continue;
                 size_t smem = 0;
                 int per_sm = 0;
@@ -2777,12 +2849,12 @@ int grlbm_batch_autotune(grlbm_batch *b, int32_t trial_steps, int32_t *blocks_pe
                 if (rc)
                     break;
                 if (ms < best)
-                    best = ms, bx = t[0], by = t[1];
+                    best = ms, bx = t[0], by = t[1], block = false;
             }
             if (rc)
                 break;
             for (grlbm_ctx *c : cls.second)
-                if ((rc = set_step32_tile(c, bx, by)))
+                if ((rc = set_step32_tile(c, bx, by)) || (block && (rc = set_block_step(c))))
                     break;
             if (rc)
                 break;

@@ -50,6 +50,7 @@
 #include <type_traits>
 
 #include "device_common.cuh"
+#include "step_block.cuh"
 #include "step_common.cuh"
 
 // resident blocks per SM the single-problem kernel is compiled for: three
@@ -60,6 +61,12 @@
 #endif
 #ifndef GRLBM_STEP32_MIN_BLOCKS_1
 #define GRLBM_STEP32_MIN_BLOCKS_1 3
+#endif
+
+// resident blocks per SM the one-patch-per-block step is compiled for (3: 80
+// registers)
+#ifndef GRLBM_BLOCK32_MIN_BLOCKS
+#define GRLBM_BLOCK32_MIN_BLOCKS 3
 #endif
 
 namespace grlbm
@@ -872,6 +879,163 @@ __global__ void __launch_bounds__(kThreads, GRLBM_STEP32_MIN_BLOCKS)
 
 inline unsigned nblk(int64_t n, int b) { return (unsigned)((n + b - 1) / b); }
 
+// The precision form in the one-patch-per-block step (step_block.cuh).
+struct Form32
+{
+    using T = float;
+    using T2 = float2;
+    using T4 = float4;
+    using Args = Step32Args;
+    using Table = DirTable;
+    static constexpr int kRow = 12; // a row type's values in shared memory
+    static constexpr int kWide = 4; // directions of a 16-byte store
+    using Rec = uint4;
+    static __device__ __forceinline__ Rec load(const Rec *p, bool ok) { return ok ? __ldcs(p) : make_uint4(0u, 0u, 0u, 0u); }
+    static constexpr int kMinBlocks = GRLBM_BLOCK32_MIN_BLOCKS;
+    static __device__ __forceinline__ float fma(float x, float y, float z) { return fmaf(x, y, z); }
+    // sqrt(sum ((prev - m) / m)^2) > 1e-4, with the fast quotient (the FP32
+    // form's choice: a noise moment near zero would otherwise take the IEEE
+    // division's slow path; 0 / 0 is still NaN).  The root is not taken: the
+    // constant is the largest float whose square root rounds to at most 1e-4f.
+    static __device__ __forceinline__ bool changing(const float (&prev)[6], const float (&m)[6])
+    {
+        float s2 = 0.f;
+#pragma unroll
+        for (int q = 0; q < 6; q++)
+        {
+            const float x = __fdividef(prev[q] - m[q], m[q]);
+            s2 += x * x;
+        }
+        return s2 > 0x1.5798eep-27f;
+    }
+    static __device__ __forceinline__ void coeffs(float n1, float n2, float u1, float u2, float lor, float adt,
+                                                  float kak0, float &g, float &h, float &q1, float &q2)
+    {
+        collide_coeffs32(n1, n2, u1, u2, lor, adt, kak0, g, h, q1, q2);
+    }
+    // one streamed value from the cell's patch (cellp: node (i - 1, j - 1))
+    static __device__ __forceinline__ float curved(const Rec &r, const float *cellp, int dps, int pdp,
+                                                   const float *rowtab, bool &far)
+    {
+        far = (r.w >> 31) != 0;
+        const unsigned word = r.x;
+        const float t = (float)(word & ((1u << packed32::kTBits) - 1u)) * (1.f / (float)(1u << packed32::kTBits));
+        const float4 *row = reinterpret_cast<const float4 *>(rowtab + ((word >> packed32::kTypeShift) & 31u) * kRow);
+        const float4 R0 = row[0], R1 = row[1], R2 = row[2];
+        const float w0 = fmaf(t, R1.x, R0.x), w1 = fmaf(t, R1.y, R0.y), w2 = fmaf(t, R1.z, R0.z);
+        const float w3 = fmaf(t, R1.w, R0.w), w4 = fmaf(t, R2.y, R2.x);
+        const int s = (int)((word >> packed32::kStartShift) & 255u);
+        const float *p00 = cellp + (int)(r.y >> 31) * dps + (int)(r.z >> 31) * pdp + s;
+        const float c00 = window5(p00, w0, w1, w2, w3, w4);
+        const float c10 = window5(p00 + dps, w0, w1, w2, w3, w4);
+        const float c01 = window5(p00 + pdp, w0, w1, w2, w3, w4);
+        const float c11 = window5(p00 + pdp + dps, w0, w1, w2, w3, w4);
+        const float fx = __uint_as_float(r.y & 0x7fffffffu), fy = __uint_as_float(r.z & 0x7fffffffu);
+        const float f0 = fmaf(fx, c10 - c00, c00);
+        const float f1 = fmaf(fx, c11 - c01, c01);
+        return __uint_as_float(r.w & 0x7fffffffu) * fmaf(fy, f1 - f0, f0);
+    }
+    static __device__ __forceinline__ float far_curved(const Args &a, const Table &dt, int i, int j,
+                                                       int cell, int d)
+    {
+        return stream_far32(a.Iin, __ldg(a.side + (unsigned)cell * (unsigned)a.nd + (unsigned)d), a.dp, (int)a.g.nx,
+                            (int)a.g.ny, a.nd, a.ng, dt.rowtab, dt.q, dt.p, dt.inv_q, i, j);
+    }
+    // a flat departure per direction: fractions, and the corner's offset in
+    // nodes {x, y} (x < 0: more than a cell away)
+    static constexpr int kFlatBytesPerDir = 16;
+    static int flat_bytes(int nd, int) { return kFlatBytesPerDir * nd; }
+    static __device__ __forceinline__ void flat_tables(const Args &a, const BlockStep &, const Table &dt,
+                                                       unsigned char *tab, int, int)
+    {
+        for (int d = threadIdx.x; d < a.nd; d += block::kThreads)
+        {
+            const float ox = dt.ox[d], oy = dt.oy[d];
+            const float fli = floorf(ox), flj = floorf(oy);
+            const bool near = (fli == -1.f || fli == 0.f) && (flj == -1.f || flj == 0.f);
+            reinterpret_cast<float4 *>(tab)[d] =
+                make_float4(ox - fli, oy - flj, __int_as_float(near ? (int)fli + 1 : -1),
+                            __int_as_float(near ? (int)flj + 1 : 0));
+        }
+    }
+    static __device__ __forceinline__ void flat_run(const Args &a, const BlockStep &, const Table &dt,
+                                                    const unsigned char *tab, const float *cellp, float *S, int n,
+                                                    int dps, int pdp, int ss, int, int, int i, int j, int d)
+    {
+        const float4 f = reinterpret_cast<const float4 *>(tab)[d];
+        const int ci = __float_as_int(f.z), cj = __float_as_int(f.w);
+        if (ci < 0)
+        {
+            for (int k = 0; k < n; k++)
+                S[k * ss] = stream_flat_far32(a.Iin, __ldg(dt.ox + d), __ldg(dt.oy + d), a.dp, (int)a.g.nx, (int)a.g.ny,
+                                              d, i + k, j);
+            return;
+        }
+        const float *p = cellp + ci * dps + cj * pdp + d;
+        float l0 = p[0], l1 = p[pdp];
+#pragma unroll 4
+        for (int k = 0; k < n; k++)
+        {
+            p += dps;
+            const float r0 = p[0], r1 = p[pdp];
+            const float f0 = fmaf(f.x, r0 - l0, l0);
+            const float f1 = fmaf(f.x, r1 - l1, l1);
+            S[k * ss] = fmaf(f.y, f1 - f0, f0);
+            l0 = r0, l1 = r1;
+        }
+    }
+    // three of the cell's moments over the directions of parity h (FP32
+    // chunks of 8 folded into Kahan sums), then both parities combined: the
+    // same sums, in the same order, as the warp-per-tile kernel's
+    static __device__ __forceinline__ void moments(const float *Sc, const float *tab, int nd, int h, unsigned lanes,
+                                                   float (&out)[3])
+    {
+        float ks[3] = {0.f, 0.f, 0.f}, kc[3] = {0.f, 0.f, 0.f};
+        for (int d0 = h; d0 < nd; d0 += 16)
+        {
+            float pp[3] = {0.f, 0.f, 0.f};
+            if (d0 + 14 < nd)
+            {
+#pragma unroll
+                for (int kk = 0; kk < 8; kk++)
+                {
+                    const float v = Sc[d0 + 2 * kk];
+                    const float4 cf = *reinterpret_cast<const float4 *>(tab + 8 * (d0 + 2 * kk));
+                    pp[0] = fmaf(cf.x, v, pp[0]);
+                    pp[1] = fmaf(cf.y, v, pp[1]);
+                    pp[2] = fmaf(cf.z, v, pp[2]);
+                }
+            }
+            else
+                for (int dd = d0; dd < nd; dd += 2)
+                {
+                    const float v = Sc[dd];
+                    const float4 cf = *reinterpret_cast<const float4 *>(tab + 8 * dd);
+                    pp[0] = fmaf(cf.x, v, pp[0]);
+                    pp[1] = fmaf(cf.y, v, pp[1]);
+                    pp[2] = fmaf(cf.z, v, pp[2]);
+                }
+#pragma unroll
+            for (int q = 0; q < 3; q++)
+            {
+                const float y = pp[q] - kc[q];
+                const float t = ks[q] + y;
+                kc[q] = (t - ks[q]) - y;
+                ks[q] = t;
+            }
+        }
+#pragma unroll
+        for (int q = 0; q < 3; q++)
+        {
+            const float os = __shfl_xor_sync(lanes, ks[q], 8), oc = __shfl_xor_sync(lanes, kc[q], 8);
+            const float x = ks[q] + os;
+            const float bp = x - ks[q];
+            const float err = (ks[q] - (x - bp)) + (os - bp);
+            out[q] = x + (err - (kc[q] + oc));
+        }
+    }
+};
+
 template <bool CURVED, int P, bool H = false>
 cudaError_t set_smem_limit()
 {
@@ -935,6 +1099,8 @@ int step32_batch_item_bytes(int q) { return (int)((sizeof(Step32Args) + sizeof(D
 
 size_t step32_batch_smem(int warp_stride) { return (size_t)kRowtabOffset + 128 + (size_t)kWarps * warp_stride; }
 
+static const void *block_kernel32(bool curved, int run);
+
 cudaError_t prepare_step32()
 {
     cudaError_t e = cudaSuccess;
@@ -952,6 +1118,10 @@ cudaError_t prepare_step32()
     GRLBM_PREP(6)
     GRLBM_PREP(8)
 #undef GRLBM_PREP
+    for (int run = 4; run <= 8; run += 4)
+        for (int curved = 0; curved < 2 && e == cudaSuccess; curved++)
+            e = cudaFuncSetAttribute(block_kernel32(curved != 0, run), cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     kStep32MaxSmem);
     if (e == cudaSuccess)
         e = set_smem_limit<true, 1, true>();
     if (e == cudaSuccess)
@@ -1013,6 +1183,34 @@ void launch_step32(const Step32Args &a, const DirTable &dt, bool curved, int P, 
     GRLBM_LAUNCH(6)
     GRLBM_LAUNCH(8)
 #undef GRLBM_LAUNCH
+}
+
+void block_layout32(BlockStep &b, int nd, int dp, int q, bool curved)
+{
+    block::set_layout<Form32>(b, nd, step32_patch_node_floats(dp), q, curved, Form32::flat_bytes(nd, b.run));
+}
+
+static const void *block_kernel32(bool curved, int run)
+{
+    if (run == 4)
+        return curved ? (const void *)block::k_step_block<Form32, true, 4>
+                      : (const void *)block::k_step_block<Form32, false, 4>;
+    return curved ? (const void *)block::k_step_block<Form32, true, 8>
+                  : (const void *)block::k_step_block<Form32, false, 8>;
+}
+
+cudaError_t block_occupancy32(bool curved, int run, int smem, int *blocks)
+{
+    return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks, block_kernel32(curved, run), block::kThreads, smem);
+}
+
+void launch_step_block32(const Step32Args &a, const BlockStep &b, const DirTable *dt, bool curved, cudaStream_t s)
+{
+    if (b.tiles_x <= 0 || b.tiles_y <= 0)
+        return;
+    void *args[] = {const_cast<Step32Args *>(&a), const_cast<BlockStep *>(&b), &dt};
+    cudaLaunchKernel(block_kernel32(curved, b.run), dim3(b.tiles_x, b.tiles_y), dim3(block::kThreads), args,
+                     (size_t)b.smem, s);
 }
 
 void launch_step_batch32(const Batch32Item *items, const int *first_tile, int n_items, int total_tiles, int flip,

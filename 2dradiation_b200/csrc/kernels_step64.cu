@@ -34,6 +34,7 @@
 #include <algorithm>
 
 #include "device_common.cuh"
+#include "step_block.cuh"
 #include "step_common.cuh"
 
 // resident blocks per SM the step is compiled for: three at one pass (at
@@ -44,6 +45,12 @@
 #endif
 #ifndef GRLBM_STEP64_MIN_BLOCKS_1
 #define GRLBM_STEP64_MIN_BLOCKS_1 3
+#endif
+
+// resident blocks per SM the one-patch-per-block step is compiled for (2: 128
+// registers)
+#ifndef GRLBM_BLOCK64_MIN_BLOCKS
+#define GRLBM_BLOCK64_MIN_BLOCKS 2
 #endif
 
 namespace grlbm
@@ -601,6 +608,161 @@ __global__ void __launch_bounds__(kThreads, P == 1 ? GRLBM_STEP64_MIN_BLOCKS_1 :
 
 inline unsigned nblk(int64_t n, int b) { return (unsigned)((n + b - 1) / b); }
 
+// The fast FP64 form in the one-patch-per-block step (step_block.cuh).
+struct Form64
+{
+    using T = double;
+    using T2 = double2;
+    using T4 = double4;
+    using Args = Step64Args;
+    using Table = DirTable64;
+    static constexpr int kRow = 10; // a row type's values in shared memory
+    static constexpr int kWide = 2; // directions of a 16-byte store
+    using Rec = double4;
+    static __device__ __forceinline__ Rec load(const Rec *p, bool ok) { return ok ? ld_once(p) : make_double4(0, 0, 0, 0); }
+    static constexpr int kMinBlocks = GRLBM_BLOCK64_MIN_BLOCKS;
+    static __device__ __forceinline__ double fma(double x, double y, double z) { return ::fma(x, y, z); }
+    // sqrt(sum ((prev - m) / m)^2) > 1e-4, the reference's relative change (0
+    // / 0 is NaN and ends the iteration).  The sum is first taken in FP32
+    // (within 1e-5 of itself while every moment is in FP32's range); only where
+    // it is within 0.1% of the limit, or not in range, are the six quotients
+    // and the root taken in FP64.
+    static __device__ __forceinline__ bool changing(const double (&prev)[6], const double (&m)[6])
+    {
+        float s = 0.f, lo = 1e30f, hi = 0.f;
+#pragma unroll
+        for (int q = 0; q < 6; q++)
+        {
+            const float d = (float)(prev[q] - m[q]), f = (float)m[q], x = __fdividef(d, f);
+            s += x * x;
+            lo = fminf(lo, fabsf(f));
+            hi = fmaxf(hi, fabsf(f));
+            // a difference below FP32's normal range counts as out of range, zero does not
+            if (d != 0.f && fabsf(d) < 1e-30f)
+                lo = 0.f;
+        }
+        if (lo > 1e-30f && hi < 1e30f && (s > 1.001e-8f || s < 0.999e-8f) && s < 1e30f)
+            return s > 1e-8f;
+        double s2 = 0.0;
+        for (int q = 0; q < 6; q++)
+        {
+            const double x = (prev[q] - m[q]) / m[q];
+            s2 += x * x;
+        }
+        return ::sqrt(s2) > 1e-4;
+    }
+    static __device__ __forceinline__ void coeffs(double n1, double n2, double u1, double u2, double lor, double adt,
+                                                  double kak0, double &g, double &h, double &q1, double &q2)
+    {
+        collide_coeffs64(n1, n2, u1, u2, lor, adt, kak0, g, h, q1, q2);
+    }
+    // one streamed value from the cell's patch (cellp: node (i - 1, j - 1))
+    static __device__ __forceinline__ double curved(const Rec &r, const double *cellp, int dps, int pdp,
+                                                    const double *rowtab, bool &far)
+    {
+        const unsigned hx = hi_word(r.x), hy = hi_word(r.y), hz = hi_word(r.z), hw = hi_word(r.w);
+        far = (hw >> 31) != 0;
+        const double fx = unbias(r.x), fy = unbias(r.y), t = unbias(r.z);
+        const double2 *row = reinterpret_cast<const double2 *>(rowtab + ((hx >> packed64::kExpShift) & 31u) * kRow);
+        const double2 R0 = row[0], R1 = row[1], R2 = row[2], R3 = row[3], R4 = row[4];
+        const double w0 = ::fma(t, R2.x, R0.x), w1 = ::fma(t, R2.y, R0.y);
+        const double w2 = ::fma(t, R3.x, R1.x), w3 = ::fma(t, R3.y, R1.y);
+        const double w4 = ::fma(t, R4.y, R4.x);
+        const int s = (int)((hz >> packed64::kExpShift) & 255u);
+        const double *p00 = cellp + (int)(hx >> 31) * dps + (int)(hy >> 31) * pdp + s;
+        const double c00 = window5(p00, w0, w1, w2, w3, w4);
+        const double c10 = window5(p00 + dps, w0, w1, w2, w3, w4);
+        const double c01 = window5(p00 + pdp, w0, w1, w2, w3, w4);
+        const double c11 = window5(p00 + pdp + dps, w0, w1, w2, w3, w4);
+        const double f0 = ::fma(fx, c10 - c00, c00);
+        const double f1 = ::fma(fx, c11 - c01, c01);
+        return __hiloint2double((int)(hw & 0x7fffffffu), __double2loint(r.w)) * ::fma(fy, f1 - f0, f0);
+    }
+    static __device__ __forceinline__ double far_curved(const Args &a, const Table &dt, int i,
+                                                        int j, int cell, int d)
+    {
+        return stream_far64(a.Iin, ld_ro(a.side + (size_t)cell * (size_t)a.nd + (size_t)d), a.dp, (int)a.g.nx,
+                            (int)a.g.ny, a.nd, a.ng, dt.rowtab, dt.q, dt.p, dt.inv_q, i, j);
+    }
+    // the flat departures' grid coordinates, per column and direction and per
+    // row and direction of the tile, rounded as the reference's xy(i, j) - c
+    // dt, then grid.i() / grid.j() (src/Radiation.cpp:394-402): a cell's two
+    // divisions per direction are shared by its column and its row
+    static int flat_bytes(int nd, int run) { return (run + kBlockStepWarps) * nd * 8; }
+    static __device__ __forceinline__ void flat_tables(const Args &a, const BlockStep &b, const Table &dt,
+                                                       unsigned char *tab, int x0, int y0)
+    {
+        double *xt = reinterpret_cast<double *>(tab), *yt = xt + b.run * a.nd;
+        for (int l = threadIdx.x >> 5; l < b.run + kBlockStepWarps; l += kBlockStepWarps)
+        {
+            const bool col = l < b.run;
+            const int ly = l - b.run;
+            const double at = col ? __dadd_rn(a.g.startx, __dmul_rn((double)(x0 + 1 + l), a.g.dx))
+                                  : __dadd_rn(a.g.starty, __dmul_rn((double)(y0 + 1 + ly), a.g.dy));
+            for (int d = threadIdx.x & 31; d < a.nd; d += 32)
+                if (col)
+                    xt[l * a.nd + d] = __ddiv_rn(__dsub_rn(__dsub_rn(at, dt.cxdt[d]), a.g.startx), a.g.dx);
+                else
+                    yt[ly * a.nd + d] = __ddiv_rn(__dsub_rn(__dsub_rn(at, dt.cydt[d]), a.g.starty), a.g.dy);
+        }
+    }
+    static __device__ __forceinline__ void flat_run(const Args &a, const BlockStep &b, const Table &,
+                                                    const unsigned char *tab, const double *cellp, double *S, int n,
+                                                    int dps, int pdp, int ss, int lx, int ly, int i, int j, int d)
+    {
+        const double *xt = reinterpret_cast<const double *>(tab) + d;
+        const double jt = xt[(b.run + ly) * a.nd];
+        const int j0 = min(max((int)floor(jt), 0), (int)a.g.ny - 2);
+        const int cj = j0 - (j - 1);
+        const double fy = jt - (double)j0;
+        const double *row = cellp + cj * pdp + d;
+        int left = -1; // the node column (from the run's first) l0 and l1 hold
+        double l0 = 0.0, l1 = 0.0;
+        for (int k = 0; k < n; k++)
+        {
+            const double it = xt[(lx + k) * a.nd];
+            const int i0 = min(max((int)floor(it), 0), (int)a.g.nx - 2);
+            const int ci = i0 - (i + k - 1);
+            if (!((unsigned)ci <= 1u && (unsigned)cj <= 1u))
+            {
+                S[k * ss] = stream_flat_far64(a.Iin, it, jt, a.dp, (int)a.g.nx, (int)a.g.ny, d);
+                left = -1;
+                continue;
+            }
+            const double *p = row + (k + ci) * dps;
+            if (left != k + ci)
+                l0 = p[0], l1 = p[pdp];
+            const double r0 = p[dps], r1 = p[dps + pdp];
+            const double fx = it - (double)i0;
+            const double f0 = ::fma(fx, r0 - l0, l0);
+            const double f1 = ::fma(fx, r1 - l1, l1);
+            S[k * ss] = ::fma(fy, f1 - f0, f0);
+            left = k + ci + 1;
+            l0 = r0, l1 = r1;
+        }
+    }
+    // three of the cell's moments over the directions of parity h, then both
+    // parities
+    static __device__ __forceinline__ void moments(const double *Sc, const double *tab, int nd, int h, unsigned lanes,
+                                                   double (&out)[3])
+    {
+        double m[3] = {0.0, 0.0, 0.0};
+#pragma unroll 4
+        for (int d = h; d < nd; d += 2)
+        {
+            const double v = Sc[d];
+            const double2 c0 = *reinterpret_cast<const double2 *>(tab + 8 * d);
+            const double c2 = tab[8 * d + 2];
+            m[0] = ::fma(c0.x, v, m[0]);
+            m[1] = ::fma(c0.y, v, m[1]);
+            m[2] = ::fma(c2, v, m[2]);
+        }
+#pragma unroll
+        for (int q = 0; q < 3; q++)
+            out[q] = m[q] + __shfl_xor_sync(lanes, m[q], 8);
+    }
+};
+
 constexpr int kPassSet[] = {1, 2, 3, 4, 6, 8};
 } // namespace
 
@@ -636,6 +798,8 @@ size_t step64_smem(int tx, int ty, int dp, int nd, int q)
            (size_t)kWarps * (size_t)step64_warp_stride(tx, ty, dp, nd);
 }
 
+static const void *block_kernel64(bool curved, int run);
+
 cudaError_t prepare_step64()
 {
     cudaError_t e = cudaSuccess;
@@ -653,6 +817,10 @@ cudaError_t prepare_step64()
     GRLBM_PREP(6)
     GRLBM_PREP(8)
 #undef GRLBM_PREP
+    for (int run = 4; run <= 8; run += 4)
+        for (int curved = 0; curved < 2 && e == cudaSuccess; curved++)
+            e = cudaFuncSetAttribute(block_kernel64(curved != 0, run), cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     kStep32MaxSmem);
     return e;
 }
 
@@ -672,6 +840,34 @@ cudaError_t step64_occupancy(int P, bool curved, size_t smem, int *blocks)
     if (!f)
         return cudaErrorInvalidValue;
     return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks, f, kThreads, smem);
+}
+
+void block_layout64(BlockStep &b, int nd, int dp, int q, bool curved)
+{
+    block::set_layout<Form64>(b, nd, step64_patch_node_elems(dp), q, curved, Form64::flat_bytes(nd, b.run));
+}
+
+static const void *block_kernel64(bool curved, int run)
+{
+    if (run == 4)
+        return curved ? (const void *)block::k_step_block<Form64, true, 4>
+                      : (const void *)block::k_step_block<Form64, false, 4>;
+    return curved ? (const void *)block::k_step_block<Form64, true, 8>
+                  : (const void *)block::k_step_block<Form64, false, 8>;
+}
+
+cudaError_t block_occupancy64(bool curved, int run, int smem, int *blocks)
+{
+    return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks, block_kernel64(curved, run), block::kThreads, smem);
+}
+
+void launch_step_block64(const Step64Args &a, const BlockStep &b, const DirTable64 *dt, bool curved, cudaStream_t s)
+{
+    if (b.tiles_x <= 0 || b.tiles_y <= 0)
+        return;
+    void *args[] = {const_cast<Step64Args *>(&a), const_cast<BlockStep *>(&b), &dt};
+    cudaLaunchKernel(block_kernel64(curved, b.run), dim3(b.tiles_x, b.tiles_y), dim3(block::kThreads), args,
+                     (size_t)b.smem, s);
 }
 
 void launch_step64(const Step64Args &a, const DirTable64 *dt, bool curved, int P, int blocks, cudaStream_t s)

@@ -49,13 +49,15 @@ __device__ __forceinline__ unsigned long long global_ns()
     return t;
 }
 // Wait for the phase of the given parity to complete, for limit_ns at most;
-// false at once when another block has already raised the fault word.  The
+// false soon when another block has already raised the fault word.  The
 // thread sleeps in the wait instruction (up to 20 us at a time) instead of
-// spinning.
+// spinning, and reads the fault word only after the first such sleep: the
+// word is in host memory, and a read over the bus takes longer than a copy
+// does to land.
 __device__ __forceinline__ bool mbar_wait(unsigned bar, unsigned parity, unsigned long long limit_ns,
                                           const unsigned *fault)
 {
-    if (mbar_test(bar, parity))
+    if (mbar_test(bar, parity) || mbar_test_sleep(bar, parity, 20000u))
         return true;
     if (fault && *reinterpret_cast<const volatile unsigned *>(fault))
         return false;
