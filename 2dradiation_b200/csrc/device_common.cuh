@@ -468,6 +468,7 @@ void launch_step_plain(const PlainStepArgs &a, bool curved, cudaStream_t s, cons
 cudaError_t run_wait_selftest(int arrive, unsigned long long limit_ns, int *completed, unsigned long long *waited_ns);
 // the adaptive streaming types in the precision form: stream, then moments
 // and collide (and the rotation update before, the halo moments after)
+cudaError_t prepare_step_prec_adaptive();
 void launch_step_prec_adaptive(const PrecStepArgs &a, const DirTable &dt, bool curved, cudaStream_t s);
 
 // The fixed streaming types in the precision form (kernels_step32.cu).

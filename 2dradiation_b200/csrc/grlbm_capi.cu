@@ -1294,6 +1294,8 @@ int grlbm_create(const grlbm_grid_desc *grid, const grlbm_metric_desc *metric, c
     }
     if (is_adaptive(ctx))
     {
+        if (ctx->fp32 && prepare_step_prec_adaptive() != cudaSuccess)
+            return fail(nullptr, GRLBM_ERR_CUDA, "cannot reserve shared memory for the adaptive step");
         // rotationAngle and rotationAngleNew start at zero (src/Radiation.cpp:3-60)
         for (auto &b : ctx->ang)
         {

@@ -148,6 +148,15 @@ __device__ __forceinline__ float intensity_at32(const PrecStepArgs &a, int n, un
     return fmaxf(fmaf(t, x1 - x0, x0), 0.f);
 }
 
+// (cos, sin) of m phi to those of (m + 1) phi, with its roundings written
+// out, so that both curved streams step alike
+__device__ __forceinline__ void next_multiple(float &cm, float &sm, float c1, float s1)
+{
+    const float c2 = __fmaf_rn(cm, c1, -__fmul_rn(sm, s1));
+    sm = __fmaf_rn(sm, c1, __fmul_rn(cm, s1));
+    cm = c2;
+}
+
 // One adaptive stream value (I, not J) of cell (i, j) for its direction d
 // rotated by the cell's new angle.  Curved streaming reads coefficient k of
 // series q of the cell at cf[q * qs + k * ks] (FP32, X and Y about the node).
@@ -179,9 +188,7 @@ __device__ __forceinline__ float stream_adaptive32(const PrecStepArgs &a, int d,
         {
             if (k & 1) // the next multiple of phi
             {
-                const float c2 = cm * c1 - sm * s1;
-                sm = sm * c1 + cm * s1;
-                cm = c2;
+                next_multiple(cm, sm, c1, s1);
             }
             const float b = sqrt2 * ((k & 1) ? cm : sm);
             const float *ck = cf + k * ks;
@@ -238,13 +245,14 @@ __global__ void __launch_bounds__(kStepBlock) k_stream_prec_adaptive_flat(PrecSt
     a.S[(size_t)d * (size_t)a.g.nxy + (size_t)ij] = stream_adaptive32<false>(a, d, i, j, ij, nullptr, 0, 0);
 }
 
-// Curved stream: a block takes 16 cells of one row for kADirs directions
+// Curved stream of small grids and many directions (below):
+// a block takes 16 cells of one row for kADirs directions
 // (16: 6% faster than 8, and 32 slower, at 400^2 x 64).
 // It first stages the row's Fourier coefficients (5 nF x 16 floats, at most
 // 20 KB) in shared memory, where its directions share them; each warp then
 // covers 16 cells x 2 directions, so a tap load reads two 16-node runs.
 constexpr int kADirs = kAdaptiveBlock / kATileX;
-__global__ void __launch_bounds__(kAdaptiveBlock) k_stream_prec_adaptive_curved(PrecStepArgs a)
+__global__ void __launch_bounds__(kAdaptiveBlock) k_stream_prec_adaptive_rows(PrecStepArgs a)
 {
     extern __shared__ float sco[]; // [q * nF + k][cell]
     // blockIdx.x: direction group fastest, then the row; blockIdx.y: the run of 16 cells
@@ -269,6 +277,195 @@ __global__ void __launch_bounds__(kAdaptiveBlock) k_stream_prec_adaptive_curved(
     if (!(a.flags[ij] & 2))
         v = stream_adaptive32<true>(a, d, i, j, ij, sco + c, kATileX, a.nf * kATileX);
     a.S[(size_t)d * (size_t)a.g.nxy + (size_t)ij] = v;
+}
+
+// Curved stream of larger grids: a block takes 32 x 2 cells with all their directions.  It
+// first copies the tile's 36 x 4 nodes of the state ([direction][row][node],
+// directions 0..3 again after the last, so that a node's 5-direction window
+// is 5 reads at fixed offsets), the interpolation rows, the nodes' rotations
+// and the cells' Fourier coefficients into shared memory.  A thread then takes
+// two directions of its cell at a time, which share the coefficient reads.
+//
+// What bound the gather from global memory (16 cells x 16 directions a block,
+// 8 tap loads and 4 row loads per corner) was the address arithmetic and the
+// loads' wavefronts: 800 instructions per 32 values, issue 70% and L1 74%
+// busy.  256^2 x 64, nF = 9: a step of 169 to
+// 139 us.
+constexpr int kAPatchX = 32, kAPatchY = 2, kAPatchCells = kAPatchX * kAPatchY;
+constexpr int kAPatchDirs = 4, kAPatchThreads = kAPatchCells * kAPatchDirs; // direction pairs in flight per cell
+// (rows of whole 16-byte copies; a plane is a multiple of the 32 banks, so
+// that lanes whose windows start at different directions still read the banks
+// of their own nodes)
+constexpr int kAPatchPitch = kAPatchX + 4, kAPatchRows = kAPatchY + 2;
+constexpr int kAPatchPlane = (kAPatchPitch * kAPatchRows + 31) / 32 * 32;
+__host__ __device__ constexpr size_t apatch_rows_at(int nd) { return (size_t)(nd + 4) * kAPatchPlane * 4; }
+__host__ __device__ constexpr size_t apatch_smem(int nd, int ng, int nf)
+{
+    return apatch_rows_at(nd) + (size_t)ng * 20 + kAPatchPitch * kAPatchRows * 8 + (size_t)5 * nf * kAPatchCells * 4;
+}
+// two blocks an SM (100 directions with 16 harmonics), and more tiles than
+// SMs; else the rows kernel, whose many short blocks fill the chip (a step of
+// 90^2 x 96, 135 tiles: 77 us with it against 86; 33 x 47 x 17: 35.5 against
+// 39; 100 x 90 x 20, 180 tiles: the same; 151 x 170 x 33, 425 tiles: 65 against 55)
+constexpr size_t kAPatchMaxSmem = 112 * 1024;
+constexpr unsigned kAPatchMinTiles = 200;
+__global__ void __launch_bounds__(kAPatchThreads, 3) k_stream_prec_adaptive_curved(const __grid_constant__ PrecStepArgs a)
+{
+    extern __shared__ __align__(16) unsigned char smem[];
+    const int nd = a.nd, ng = a.ng, nf = a.nf, nx = (int)a.g.nx, ny = (int)a.g.ny;
+    float *patch = reinterpret_cast<float *>(smem);
+    float4 *wrow = reinterpret_cast<float4 *>(smem + apatch_rows_at(nd));
+    float2 *rot = reinterpret_cast<float2 *>(wrow + ng);
+    int *brow = reinterpret_cast<int *>(rot + kAPatchPitch * kAPatchRows); // 2 first direction + (the next row starts one on)
+    float *co = reinterpret_cast<float *>(brow + ng);                      // [series * nF + k][cell]
+    const int t = threadIdx.x, cell = t % kAPatchCells, lx = t % kAPatchX, ly = (t / kAPatchX) % kAPatchY;
+    const int x0 = (int)blockIdx.x * kAPatchX, y0 = (int)a.g.jlo - 1 + (int)blockIdx.y * kAPatchY; // the patch's first node
+    const int i = x0 + 1 + lx, j = y0 + 1 + ly, ij = i + j * nx;
+    const bool active = i <= (int)a.g.nx_ && j < (int)a.g.jhi;
+    {
+        constexpr int kQuads = kAPatchPitch / 4, kPerPlane = kQuads * kAPatchRows;
+        for (int e = t; e < (nd + 4) * kPerPlane; e += kAPatchThreads)
+        {
+            const int p = e / kPerPlane, r = (e - p * kPerPlane) / kQuads, c4 = 4 * (e % kQuads);
+            const int d = p < nd ? p : (p - nd) % nd;
+            if (x0 + c4 < (int)a.pitch && y0 + r < ny) // (a row's pitch is a multiple of 4)
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(
+                                 smem_addr(patch + p * kAPatchPlane + r * kAPatchPitch + c4)),
+                             "l"(a.Iin + ((unsigned)d * a.plane + (unsigned)(y0 + r) * a.pitch + (unsigned)(x0 + c4)))
+                             : "memory");
+        }
+    }
+    for (int g = t; g < ng; g += kAPatchThreads)
+    {
+        const IgRow32 *r0 = a.ig_rows + g, *r1 = a.ig_rows + (g + 1 == ng ? 0 : g + 1);
+        wrow[g] = r0->w;
+        brow[g] = 2 * r0->idx.x + (r1->idx.x != r0->idx.x);
+    }
+    for (int n = t; n < kAPatchPitch * kAPatchRows; n += kAPatchThreads)
+    {
+        const int ni = x0 + n % kAPatchPitch, nj = y0 + n / kAPatchPitch;
+        if (ni < nx && nj < ny)
+            rot[n] = a.rot_inv[ni + nj * nx];
+    }
+    // coefficient k of series q of node ij sits at coef32[(q nF + k) nxy + ij]
+    if (active)
+        for (int p = t / kAPatchCells; p < 5 * nf; p += kAPatchDirs)
+            co[p * kAPatchCells + cell] = a.coef32[(size_t)p * (size_t)a.g.nxy + (size_t)ij];
+    asm volatile("cp.async.wait_all;\n" ::: "memory");
+    __syncthreads();
+    if (!active)
+        return;
+    float *S = a.S + ij;
+    if (a.flags[ij] & 2)
+    {
+        for (int d = t / kAPatchCells; d < nd; d += kAPatchDirs)
+            S[(size_t)d * (size_t)a.g.nxy] = 0.f;
+        return;
+    }
+    const float2 rn = a.rot_new[ij];
+    const float sc = rn.x, cc = rn.y, ia3 = a.ia3[ij];
+    const float *cf = co + cell;
+    const int qs = nf * kAPatchCells;
+    for (int d0 = 2 * (t / kAPatchCells); d0 < nd; d0 += 2 * kAPatchDirs)
+    {
+        // the five series (S, X - x, Y - y, Cx, Cy) at the directions' angles:
+        // basis {1, sqrt2 cos(m phi), sqrt2 sin(m phi)} from one sincos and
+        // the angle-addition recurrence
+        float r[2][5], s1[2], c1[2], cm[2] = {1.f, 1.f}, sm[2] = {0.f, 0.f};
+#pragma unroll
+        for (int u = 0; u < 2; u++)
+        {
+            const int d = min(d0 + u, nd - 1);
+            const float cxd = a.cx[d], cyd = a.cy[d];
+            const float dir1 = cxd * cc - cyd * sc, dir2 = cxd * sc + cyd * cc;
+            sincosf(grid_row_of(dir1, dir2, 1.f), &s1[u], &c1[u]);
+#pragma unroll
+            for (int q = 0; q < 5; q++)
+                r[u][q] = cf[q * qs];
+        }
+        const float sqrt2 = 1.41421356237f;
+        for (int k = 1; k < nf; k++)
+        {
+            float b[2];
+#pragma unroll
+            for (int u = 0; u < 2; u++)
+            {
+                if (k & 1) // the next multiple of phi
+                {
+                    next_multiple(cm[u], sm[u], c1[u], s1[u]);
+                }
+                b[u] = sqrt2 * ((k & 1) ? cm[u] : sm[u]);
+            }
+            const float *ck = cf + k * kAPatchCells;
+#pragma unroll
+            for (int q = 0; q < 5; q++)
+            {
+                const float x = ck[q * qs];
+                r[0][q] = fmaf(x, b[0], r[0][q]);
+                r[1][q] = fmaf(x, b[1], r[1][q]);
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < 2; u++)
+        {
+            if (d0 + u >= nd)
+                break;
+            float val = 0.f;
+            // the departure point, absolute for the excision test
+            const double xt = a.g.startx + (double)i * a.g.dx + (double)r[u][1];
+            const double yt = a.g.starty + (double)j * a.g.dy + (double)r[u][2];
+            if (!dev_inside_bh(a.g, xt, yt))
+            {
+                const float it = (float)i + r[u][1] * a.inv_dx, jt = (float)j + r[u][2] * a.inv_dy;
+                const float sh = r[u][0], v1 = r[u][3], v2 = r[u][4];
+                const float s3 = sh * sh * sh;
+                const int i0 = min(max((int)floorf(it), 0), nx - 2);
+                const int j0 = min(max((int)floorf(jt), 0), ny - 2);
+                const float fx = it - (float)i0, fy = jt - (float)j0;
+                float Iq[4];
+                if ((unsigned)(i0 - i + 1) <= 1u && (unsigned)(j0 - j + 1) <= 1u)
+                {
+#pragma unroll
+                    for (int q = 0; q < 4; q++) // corners 00, 01, 10, 11 (intensity_at32 from the patch)
+                    {
+                        const int n = (i0 - x0 + (q >> 1)) + (j0 - y0 + (q & 1)) * kAPatchPitch;
+                        const float2 rinv = rot[n];
+                        const float w1 = v1 * rinv.y - v2 * rinv.x, w2 = v1 * rinv.x + v2 * rinv.y;
+                        float dd = grid_row_of(w1, w2, (float)ng * 0.159154943091895f);
+                        dd = fminf(fmaxf(dd, 1e-8f), nextafterf((float)ng, 0.f));
+                        const int g0 = min((int)dd, ng - 1), g1 = g0 + 1 == ng ? 0 : g0 + 1;
+                        const float tt = dd - (float)g0;
+                        const float4 wa = wrow[g0], wb = wrow[g1];
+                        const int bs = brow[g0];
+                        const float *p = patch + ((bs >> 1) * kAPatchPlane + n);
+                        const float y0_ = p[0], y1 = p[kAPatchPlane], y2 = p[2 * kAPatchPlane], y3 = p[3 * kAPatchPlane],
+                                    y4 = p[4 * kAPatchPlane];
+                        const bool shift = bs & 1;
+                        const float xa = fmaf(wa.w, y3, fmaf(wa.z, y2, fmaf(wa.y, y1, fmaf(wa.x, y0_, 0.f))));
+                        const float xb = fmaf(wb.w, shift ? y4 : y3,
+                                              fmaf(wb.z, shift ? y3 : y2,
+                                                   fmaf(wb.y, shift ? y2 : y1, fmaf(wb.x, shift ? y1 : y0_, 0.f))));
+                        Iq[q] = fmaxf(fmaf(tt, xb - xa, xa), 0.f);
+                    }
+                }
+                else
+#pragma unroll 1
+                    for (int q = 0; q < 4; q++)
+                    {
+                        const int ci = i0 + (q >> 1), cj = j0 + (q & 1);
+                        const float v = intensity_at32(a, ci + cj * nx, (unsigned)ci + (unsigned)cj * a.pitch, v1, v2);
+                        Iq[0] = q == 0 ? v : Iq[0], Iq[1] = q == 1 ? v : Iq[1];
+                        Iq[2] = q == 2 ? v : Iq[2], Iq[3] = q == 3 ? v : Iq[3];
+                    }
+                const float f0 = fmaf(fx, Iq[2] - Iq[0], Iq[0]);
+                const float f1 = fmaf(fx, Iq[3] - Iq[1], Iq[1]);
+                const float bil = fmaf(fy, f1 - f0, f0);
+                // corners hold J = I / alpha^3: (alpha_ij / alpha_c)^3 I_c = alpha_ij^3 J_c
+                val = s3 * bil / ia3;
+            }
+            S[(size_t)(d0 + u) * (size_t)a.g.nxy] = val;
+        }
+    }
 }
 
 // Moments and collide of one cell from its streamed values, with its
@@ -554,6 +751,12 @@ void launch_coef_about_node32(const GridDev &g, const double *coef, float *coef3
     k_coef_about_node32<<<nblk(5 * g.nxy * nf, 256), 256, 0, s>>>(g, coef, coef32, nf);
 }
 
+cudaError_t prepare_step_prec_adaptive()
+{
+    return cudaFuncSetAttribute(k_stream_prec_adaptive_curved, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                (int)kAPatchMaxSmem);
+}
+
 void launch_step_prec_adaptive(const PrecStepArgs &a, const DirTable &dt, bool curved, cudaStream_t s)
 {
     const int64_t rows = a.g.jhi - a.g.jlo;
@@ -567,9 +770,16 @@ void launch_step_prec_adaptive(const PrecStepArgs &a, const DirTable &dt, bool c
     const dim3 cgrid(tx, ty);
     if (curved)
     {
-        const dim3 sgrid(nblk(a.nd, kADirs) * (unsigned)rows, tx);
-        const size_t coef_bytes = (size_t)5 * a.nf * kATileX * sizeof(float);
-        k_stream_prec_adaptive_curved<<<sgrid, kAdaptiveBlock, coef_bytes, s>>>(a);
+        const size_t smem = apatch_smem(a.nd, a.ng, a.nf);
+        const dim3 tiles(nblk(a.g.nx_, kAPatchX), nblk(rows, kAPatchY));
+        if (smem <= kAPatchMaxSmem && tiles.x * tiles.y >= kAPatchMinTiles)
+            k_stream_prec_adaptive_curved<<<tiles, kAPatchThreads, smem, s>>>(a);
+        else
+        {
+            const dim3 sgrid(nblk(a.nd, kADirs) * (unsigned)rows, tx);
+            const size_t coef_bytes = (size_t)5 * a.nf * kATileX * sizeof(float);
+            k_stream_prec_adaptive_rows<<<sgrid, kAdaptiveBlock, coef_bytes, s>>>(a);
+        }
         k_collide_prec_adaptive<true><<<cgrid, kStepBlock, 0, s>>>(a, dt);
     }
     else
