@@ -265,7 +265,7 @@ class Radiation:
         self._c(lib().grlbm_set_intensity(self.h, _p(I)))
 
     def intensity(self) -> np.ndarray:
-        out = np.zeros(self.nxy * self.nd)
+        out = np.empty(self.nxy * self.nd)
         self._c(lib().grlbm_get_intensity(self.h, _p(out)))
         return out
 
@@ -300,13 +300,13 @@ class Radiation:
 
     def moments_if(self, out: dict | None = None) -> dict:
         names = ("E", "Fx", "Fy", "Pxx", "Pxy", "Pyy")
-        out = out if out is not None else {k: np.zeros(self.nxy) for k in names}
+        out = out if out is not None else {k: np.empty(self.nxy) for k in names}
         self._c(lib().grlbm_get_moments_if(self.h, *[_p(out[k]) for k in names]))
         return out
 
     def moments_lf(self) -> dict:
         names = ("E_LF", "Fx_LF", "Fy_LF", "Pxx_LF", "Pxy_LF", "Pyy_LF", "F_LF")
-        out = {k: np.zeros(self.nxy) for k in names}
+        out = {k: np.empty(self.nxy) for k in names}
         self._c(lib().grlbm_compute_moments_lf(self.h, *[_p(out[k]) for k in names]))
         return out
 
