@@ -25,9 +25,9 @@
 // to 39 and 92 to 67 us; 200^2 x 32 20.4 to 16.3 and 34.7 to 28.1 us; flat 300^2
 // x 64 31.1 to 28.8 and 98 to 56 us; 100^2 x 20 9.3 to 7.2 and 15.3 to 10.2 us.
 //
-// What bounds it at 400^2 x 64: in FP32 instruction issue (64% busy, 67 M warp
+// What bounds it at 400^2 x 64: in FP32 instruction issue (67% busy, 66 M warp
 // instructions) and shared-memory reads (71% of the wavefronts); in FP64 the
-// shared-memory reads (76%).  Tried and left out, at that size: a persistent
+// shared-memory reads (68%) and the chains of 16 warps.  Tried and left out, at that size: a persistent
 // grid with the next patch staged during phases 2 and 3 (FP32 96 us: registers
 // spill), and a lane per direction along the run in curved streaming too, its
 // taps and weights kept for the next cell where the window and corner stay (91

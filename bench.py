@@ -603,9 +603,9 @@ def run_grlbm(a, world, rank, local, pg):
             "peak_kind": peak_kind,
             "unit": "GB/s",
             "frac": ach32 / peak,
-            "traffic": profiled_traffic("k_step_prec"),
+            "traffic": profiled_traffic("k_step_block32"),
             "algorithmic_bytes_per_update": b32,
-            "kernel": "k_step_prec<curved>",
+            "kernel": "k_step_block<FP32, curved>",
         },
         "plain_fp64": {
             "value": plain,
@@ -622,8 +622,8 @@ def run_grlbm(a, world, rank, local, pg):
             "roofline_frac": achf / peak,
             "achieved_gbs": achf,
             "algorithmic_bytes_per_update": b64,
-            "traffic": profiled_traffic("k_step_fast64"),
-            "kernel": "k_step_fast64<curved> (FP64, contracted FMAs, 32-byte packed records; matches the "
+            "traffic": profiled_traffic("k_step_block64"),
+            "kernel": "k_step_block<FP64, curved> (FP64, contracted FMAs, 32-byte packed records; matches the "
                       "reference to 1e-12 where the lambda iteration's cycle count is not set by rounding noise)",
             "accuracy": fast_accuracy,
             "e2e": e2e_line("fast64"),
