@@ -250,14 +250,30 @@ int alloc(grlbm_ctx *ctx, DevBuf &b, size_t bytes)
     return GRLBM_OK;
 }
 
+// Device memory is written on the stream of the kernels that read it, never
+// on the default stream: the contexts' streams do not wait for that one, and
+// a plain cudaMemcpy from pageable memory (or cudaMemset) may return before
+// its data has landed.  The wait here is for the host's vector.
+template <class T>
+int upload(grlbm_ctx *ctx, DevBuf &b, const std::vector<T> &v, cudaStream_t stream)
+{
+    int rc = alloc(ctx, b, v.size() * sizeof(T));
+    if (rc || v.empty())
+        return rc;
+    CU(cudaMemcpyAsync(b.p, v.data(), v.size() * sizeof(T), cudaMemcpyHostToDevice, stream));
+    CU(cudaStreamSynchronize(stream));
+    return GRLBM_OK;
+}
 template <class T>
 int upload(grlbm_ctx *ctx, DevBuf &b, const std::vector<T> &v)
 {
-    int rc = alloc(ctx, b, v.size() * sizeof(T));
-    if (rc)
-        return rc;
-    if (!v.empty())
-        CU(cudaMemcpy(b.p, v.data(), v.size() * sizeof(T), cudaMemcpyHostToDevice));
+    return upload(ctx, b, v, ctx->stream);
+}
+
+int zero(grlbm_ctx *ctx, DevBuf &b)
+{
+    if (b.p)
+        CU(cudaMemsetAsync(b.p, 0, b.bytes, ctx->stream));
     return GRLBM_OK;
 }
 
@@ -1351,7 +1367,7 @@ int grlbm_create(const grlbm_grid_desc *grid, const grlbm_metric_desc *metric, c
     else
     {
         TRY(alloc(ctx, ctx->acube, (size_t)nxy * 9 * sizeof(double)));
-        cudaMemset(ctx->acube.p, 0, ctx->acube.bytes);
+        TRY(zero(ctx, ctx->acube));
         launch_alpha_cube(gd, ctx->alpha.as<double>(), ctx->acube.as<double>(), ctx->stream);
     }
 
@@ -1397,11 +1413,11 @@ int grlbm_create(const grlbm_grid_desc *grid, const grlbm_metric_desc *metric, c
         TRY(alloc(ctx, ctx->rec, (size_t)ctx->ncell * nd * sizeof(double4)));
     TRY(alloc(ctx, ctx->counters, 8 * sizeof(unsigned long long)));
     TRY(alloc(ctx, ctx->tile_ctr, 2 * sizeof(unsigned)));
-    cudaMemset(ctx->tile_ctr.p, 0, ctx->tile_ctr.bytes);
+    TRY(zero(ctx, ctx->tile_ctr));
     TRY(alloc(ctx, ctx->energy_partial, kPartialBlocks * sizeof(double)));
     TRY(alloc(ctx, ctx->energy_out, sizeof(double)));
-    cudaMemset(ctx->I[0].p, 0, ib);
-    cudaMemset(ctx->I[1].p, 0, ib);
+    TRY(zero(ctx, ctx->I[0]));
+    TRY(zero(ctx, ctx->I[1]));
     if (is_tiled(ctx))
     {
         ctx->passes = ctx->fast64 ? step64_passes(nd) : step32_passes(nd);
@@ -1419,7 +1435,7 @@ int grlbm_create(const grlbm_grid_desc *grid, const grlbm_metric_desc *metric, c
         for (auto &b : ctx->ang)
         {
             TRY(alloc(ctx, b, (size_t)nxy * sizeof(double)));
-            cudaMemset(b.p, 0, b.bytes);
+            TRY(zero(ctx, b));
         }
         TRY(alloc(ctx, ctx->rot, 2 * (size_t)nxy * (ctx->fp32 ? sizeof(float2) : sizeof(double2))));
         if (ctx->fp32)
@@ -1430,16 +1446,15 @@ int grlbm_create(const grlbm_grid_desc *grid, const grlbm_metric_desc *metric, c
         }
         ctx->flux_angle.assign(nxy, 0.0);
     }
-    cudaMemset(ctx->mom.p, 0, ctx->mom.bytes);
-    cudaMemset(ctx->counters.p, 0, ctx->counters.bytes);
-    if (ctx->rec.p)
-        cudaMemset(ctx->rec.p, 0, ctx->rec.bytes);
+    TRY(zero(ctx, ctx->mom));
+    TRY(zero(ctx, ctx->counters));
+    TRY(zero(ctx, ctx->rec));
     // fields default to zero (the reference's buffers are value-initialised)
     std::vector<double> zeros(nxy, 0.0);
     TRY(grlbm_set_fields(ctx, zeros.data(), zeros.data(), zeros.data(), zeros.data(), zeros.data(), zeros.data()));
     if (!ctx->fp32 && prepare_step_plain(0) != cudaSuccess)
         return fail(nullptr, GRLBM_ERR_CUDA, "cannot reserve shared memory for the step kernel");
-    if (cudaDeviceSynchronize() != cudaSuccess)
+    if (cudaStreamSynchronize(ctx->stream) != cudaSuccess)
         return fail(nullptr, GRLBM_ERR_CUDA, "device error during set-up");
 #undef TRY
     *out = owner.release();
@@ -2602,8 +2617,9 @@ int batch_build(grlbm_batch *b)
     }
     if (alloc(nullptr, b->d_items, n * sizeof(Batch32Item)) || alloc(nullptr, b->d_first, (n + 1) * sizeof(int)))
         return bfail(b, GRLBM_ERR_CUDA, "cannot allocate the batch launch list");
-    BCU(cudaMemcpy(b->d_items.p, b->items.data(), n * sizeof(Batch32Item), cudaMemcpyHostToDevice));
-    BCU(cudaMemcpy(b->d_first.p, first.data(), (n + 1) * sizeof(int), cudaMemcpyHostToDevice));
+    BCU(cudaMemcpyAsync(b->d_items.p, b->items.data(), n * sizeof(Batch32Item), cudaMemcpyHostToDevice, b->stream));
+    BCU(cudaMemcpyAsync(b->d_first.p, first.data(), (n + 1) * sizeof(int), cudaMemcpyHostToDevice, b->stream));
+    BCU(cudaStreamSynchronize(b->stream)); // the host's lists may go
     b->flip = 0;
     batch_drop_graphs(b);
     return GRLBM_OK;
@@ -2776,11 +2792,11 @@ int grlbm_batch_create(grlbm_ctx *const *ctxs, int32_t n, grlbm_batch **out)
     BCU(cudaDeviceGetAttribute(&b->sms, cudaDevAttrMultiProcessorCount, b->device));
     if (alloc(nullptr, b->counters, 2 * sizeof(unsigned)))
         return bfail(nullptr, GRLBM_ERR_CUDA, "grlbm_batch_create: cannot allocate the tile counters");
-    BCU(cudaMemset(b->counters.p, 0, b->counters.bytes));
+    BCU(cudaMemsetAsync(b->counters.p, 0, b->counters.bytes, b->stream));
     std::vector<DirTable> dirs(n);
     for (int k = 0; k < n; k++)
         dirs[k] = ctxs[k]->dirs;
-    if (upload(nullptr, b->d_dirs, dirs))
+    if (upload(nullptr, b->d_dirs, dirs, b->stream))
         return bfail(nullptr, GRLBM_ERR_CUDA, "grlbm_batch_create: cannot upload the direction tables");
     int rc = batch_geometry(b);
     if (rc)
@@ -2862,7 +2878,7 @@ int grlbm_batch_autotune(grlbm_batch *b, int32_t trial_steps, int32_t *blocks_pe
             std::unique_ptr<DevBuf> copy(new DevBuf);
             if (alloc(nullptr, *copy, d->bytes))
                 return bfail(b, GRLBM_ERR_CUDA, "autotune: cannot allocate a state copy");
-            BCU(cudaMemcpy(copy->p, d->p, d->bytes, cudaMemcpyDeviceToDevice));
+            BCU(cudaMemcpyAsync(copy->p, d->p, d->bytes, cudaMemcpyDeviceToDevice, b->stream));
             saved.emplace_back(d, std::move(copy));
         }
     }
@@ -2965,7 +2981,8 @@ int grlbm_batch_autotune(grlbm_batch *b, int32_t trial_steps, int32_t *blocks_pe
     // restore the saved state (the trials leave every context's current
     // buffer index as it was)
     for (auto &sv : saved)
-        BCU(cudaMemcpy(sv.first->p, sv.second->p, sv.first->bytes, cudaMemcpyDeviceToDevice));
+        BCU(cudaMemcpyAsync(sv.first->p, sv.second->p, sv.first->bytes, cudaMemcpyDeviceToDevice, b->stream));
+    BCU(cudaStreamSynchronize(b->stream)); // before the contexts' own steps read it, and the copies go
     if (rc)
         return rc;
     if ((rc = batch_build(b)))
