@@ -10,7 +10,6 @@
 #include <cstdlib>
 #include <cstring>
 #include <memory>
-#include <mutex>
 #include <string>
 #include <vector>
 
@@ -19,6 +18,7 @@
 #include "device_common.cuh"
 #include "frames.hpp"
 #include "host_setup.hpp"
+#include "read_back_buffers.hpp"
 #include "runlog.hpp"
 
 using namespace grlbm;
@@ -26,40 +26,31 @@ using namespace grlbm;
 namespace
 {
 thread_local std::string g_create_error;
-// half of a context's page-locked read-back buffer
+// half of a page-locked read-back buffer
 constexpr size_t kBounceBytes = 512 * 1024;
-// Destroyed contexts leave their read-back buffers to the next ones, at most
-// this many (page-locking and unlocking one costs more than a small problem's
-// whole read-back); further ones are freed.
-constexpr size_t kBounceKept = 4;
-std::mutex g_bounce_mutex;
-std::vector<char *> g_bounce_kept;
-char *take_bounce()
-{
-    {
-        std::lock_guard<std::mutex> lock(g_bounce_mutex);
-        g_bounce_kept.reserve(kBounceKept); // giving one back never allocates
-        if (!g_bounce_kept.empty())
-        {
-            char *p = g_bounce_kept.back();
-            g_bounce_kept.pop_back();
+// (never destroyed: contexts may be, after this file's static objects)
+ReadBackBuffers &g_bounce = *new ReadBackBuffers(
+    [] {
+        char *p = nullptr;
+        if (cudaHostAlloc(reinterpret_cast<void **>(&p), 2 * kBounceBytes, cudaHostAllocPortable) == cudaSuccess)
             return p;
-        }
-    }
-    char *p = nullptr;
-    return cudaHostAlloc(reinterpret_cast<void **>(&p), 2 * kBounceBytes, cudaHostAllocPortable) == cudaSuccess ? p : nullptr;
-}
-void give_bounce(char *p)
+        cudaGetLastError(); // not an error of the call: results are then copied directly
+        return static_cast<char *>(nullptr);
+    },
+    [](char *p) { cudaFreeHost(p); });
+// the current device's CUDA context by its number; false where the driver has none to give
+bool bounce_place(int device, ReadBackBuffers::Place *at)
 {
-    {
-        std::lock_guard<std::mutex> lock(g_bounce_mutex);
-        if (g_bounce_kept.size() < kBounceKept)
-        {
-            g_bounce_kept.push_back(p);
-            return;
-        }
-    }
-    cudaFreeHost(p);
+    using Get = CUresult(CUDAAPI *)(CUcontext, unsigned long long *);
+    static const Get get = [] {
+        void *fn = nullptr;
+        cudaDriverEntryPointQueryResult q;
+        const bool ok = cudaGetDriverEntryPointByVersion("cuCtxGetId", &fn, 12000, cudaEnableDefault, &q) == cudaSuccess &&
+                        q == cudaDriverEntryPointSuccess;
+        return ok ? reinterpret_cast<Get>(fn) : nullptr;
+    }();
+    at->device = device;
+    return get && get(nullptr, &at->context) == CUDA_SUCCESS;
 }
 
 struct DevBuf
@@ -99,10 +90,7 @@ struct grlbm_ctx
     int tile_x = 4, tile_y = 4, passes = 1, step_blocks = 1;
     CUtensorMap in_map[2];
     BlockStep blk[2] = {}; // blk[k]: the one-patch-per-block step that reads buffer k (smem 0: not used)
-    // page-locked halves through which results reach pageable host memory, and
-    // the events that say a half has landed
-    char *bounce = nullptr;
-    cudaEvent_t landed[2] = {nullptr, nullptr};
+    cudaEvent_t landed[2] = {nullptr, nullptr}; // a half of a read-back buffer has landed
     unsigned *fault = nullptr; // mapped host word: a precision step's staging wait timed out
     int64_t ncell = 0;
     int ng = 0;
@@ -160,8 +148,6 @@ struct grlbm_ctx
         for (auto &g : graph)
             if (g)
                 cudaGraphExecDestroy(g);
-        if (stream && bounce)
-            cudaStreamSynchronize(stream); // nothing lands in the halves any more
         if (stream)
             cudaStreamDestroy(stream);
         if (fault)
@@ -169,8 +155,6 @@ struct grlbm_ctx
         for (cudaEvent_t e : landed)
             if (e)
                 cudaEventDestroy(e);
-        if (bounce)
-            give_bounce(bounce);
     }
 };
 
@@ -362,12 +346,23 @@ int step32_tiles(const grlbm_ctx *ctx)
     return rows <= 0 ? 0 : step32_tiles_x(ctx) * (int)((rows + ctx->tile_y - 1) / ctx->tile_y);
 }
 
+void copy_out(const double *from, int64_t n, double *to) { std::memcpy(to, from, (size_t)n * sizeof(double)); }
+// (apart, and its arguments said not to overlap, so that it is vectorised
+// wherever the read-back is inlined: 81 against 94 us for a beam step and its moments)
+__attribute__((noinline)) void copy_out(const float *__restrict__ from, int64_t n, double *__restrict__ to)
+{
+    for (int64_t k = 0; k < n; k++)
+        to[k] = from[k];
+}
+
 // Copies nq arrays of `per` values, one after another at `src` on the device,
 // to dst[q] (null: not wanted), widening to double, once the stream's work is
-// done.  Pageable destinations are reached through the context's page-locked
+// done.  Pageable destinations are reached through a page-locked buffer's
 // halves, one landing while the host empties the other: a copy from the
 // device to pageable memory is staged by the driver, call by call (the six
 // moments of a 100^2 grid: 200 against 47 us; of 400^2: 1.4 against 0.5 ms).
+// Other destinations, and all where no such buffer can be had, are copied to
+// directly.
 template <class S>
 int read_back(grlbm_ctx *ctx, const S *src, int nq, int64_t per, double *const *dst)
 {
@@ -379,7 +374,24 @@ int read_back(grlbm_ctx *ctx, const S *src, int nq, int64_t per, double *const *
             CU(cudaPointerGetAttributes(&at, dst[q]));
             pageable = at.type == cudaMemoryTypeUnregistered;
         }
-    if (!pageable)
+    // the buffer goes back when nothing lands in it any more, on every way out
+    struct Bounce
+    {
+        cudaStream_t stream;
+        ReadBackBuffers::Place at{};
+        char *p = nullptr;
+        bool landed = false;
+        ~Bounce()
+        {
+            if (p && !landed)
+                cudaStreamSynchronize(stream);
+            if (p)
+                g_bounce.give(at, p);
+        }
+    } bounce{ctx->stream};
+    if (pageable && bounce_place(ctx->device, &bounce.at))
+        bounce.p = g_bounce.take(bounce.at);
+    if (!bounce.p)
     {
         const double *from = reinterpret_cast<const double *>(src);
         if (sizeof(S) != sizeof(double))
@@ -398,7 +410,7 @@ int read_back(grlbm_ctx *ctx, const S *src, int nq, int64_t per, double *const *
         return GRLBM_OK;
     }
     const int64_t total = nq * per, chunk = (int64_t)(kBounceBytes / sizeof(S)), n_chunks = (total + chunk - 1) / chunk;
-    auto half = [&](int64_t k) { return reinterpret_cast<S *>(ctx->bounce + (k & 1) * kBounceBytes); };
+    auto half = [&](int64_t k) { return reinterpret_cast<S *>(bounce.p + (k & 1) * kBounceBytes); };
     for (int64_t k = -1; k < n_chunks; k++)
     {
         if (k + 1 < n_chunks)
@@ -415,17 +427,12 @@ int read_back(grlbm_ctx *ctx, const S *src, int nq, int64_t per, double *const *
         {
             const int64_t q = at / per, stop = std::min(end, (q + 1) * per);
             if (double *d = dst[q])
-            {
-                if (sizeof(S) == sizeof(double))
-                    std::memcpy(d + (at - q * per), h, (size_t)(stop - at) * sizeof(double));
-                else
-                    std::copy(h, h + (stop - at), d + (at - q * per));
-            }
+                copy_out(h, stop - at, d + (at - q * per));
             h += stop - at;
             at = stop;
         }
     }
-    CU(cudaStreamSynchronize(ctx->stream));
+    bounce.landed = true;
     return GRLBM_OK;
 }
 
@@ -1398,11 +1405,9 @@ int grlbm_create(const grlbm_grid_desc *grid, const grlbm_metric_desc *metric, c
             return fail(nullptr, GRLBM_ERR_CUDA, "cudaHostAlloc of the fault word failed");
         *ctx->fault = 0;
     }
-    ctx->bounce = take_bounce();
-    if (!ctx->bounce ||
-        cudaEventCreateWithFlags(&ctx->landed[0], cudaEventDisableTiming) != cudaSuccess ||
-        cudaEventCreateWithFlags(&ctx->landed[1], cudaEventDisableTiming) != cudaSuccess)
-        return fail(nullptr, GRLBM_ERR_CUDA, "cannot allocate the read-back buffer");
+    for (cudaEvent_t &e : ctx->landed)
+        if (cudaEventCreateWithFlags(&e, cudaEventDisableTiming) != cudaSuccess)
+            return fail(nullptr, GRLBM_ERR_CUDA, "cudaEventCreate failed");
     TRY(alloc(ctx, ctx->I[0], ib));
     TRY(alloc(ctx, ctx->I[1], ib));
     if ((!ctx->fp32 && !ctx->fast64) || is_adaptive(ctx))
