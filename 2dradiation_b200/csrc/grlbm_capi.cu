@@ -19,6 +19,7 @@
 #include "frames.hpp"
 #include "host_setup.hpp"
 #include "read_back_buffers.hpp"
+#include "read_back_plan.hpp"
 #include "runlog.hpp"
 
 using namespace grlbm;
@@ -362,7 +363,7 @@ __attribute__((noinline)) void copy_out(const float *__restrict__ from, int64_t 
 // device to pageable memory is staged by the driver, call by call (the six
 // moments of a 100^2 grid: 200 against 47 us; of 400^2: 1.4 against 0.5 ms).
 // Other destinations, and all where no such buffer can be had, are copied to
-// directly.
+// directly.  Only the arrays that are wanted cross the bus.
 template <class S>
 int read_back(grlbm_ctx *ctx, const S *src, int nq, int64_t per, double *const *dst)
 {
@@ -399,7 +400,9 @@ int read_back(grlbm_ctx *ctx, const S *src, int nq, int64_t per, double *const *
             int rc = alloc(ctx, ctx->lf_out, (size_t)std::max(nq, 7) * per * sizeof(double));
             if (rc)
                 return rc;
-            launch_widen32(reinterpret_cast<const float *>(src), ctx->lf_out.as<double>(), nq * per, ctx->stream);
+            ReadBackPlan(dst, nq, per, nq * per).copies(0, [&](int64_t first, int64_t n, int64_t) {
+                launch_widen32(reinterpret_cast<const float *>(src) + first, ctx->lf_out.as<double>() + first, n, ctx->stream);
+            });
             CU(cudaGetLastError());
             from = ctx->lf_out.as<double>();
         }
@@ -409,29 +412,28 @@ int read_back(grlbm_ctx *ctx, const S *src, int nq, int64_t per, double *const *
         CU(cudaStreamSynchronize(ctx->stream));
         return GRLBM_OK;
     }
-    const int64_t total = nq * per, chunk = (int64_t)(kBounceBytes / sizeof(S)), n_chunks = (total + chunk - 1) / chunk;
+    const ReadBackPlan plan(dst, nq, per, (int64_t)(kBounceBytes / sizeof(S)));
     auto half = [&](int64_t k) { return reinterpret_cast<S *>(bounce.p + (k & 1) * kBounceBytes); };
-    for (int64_t k = -1; k < n_chunks; k++)
+    for (int64_t k = -1; k < plan.chunks(); k++)
     {
-        if (k + 1 < n_chunks)
+        if (k + 1 < plan.chunks())
         {
-            const int64_t first = (k + 1) * chunk, n = std::min(chunk, total - first);
-            CU(cudaMemcpyAsync(half(k + 1), src + first, n * sizeof(S), cudaMemcpyDeviceToHost, ctx->stream));
+            cudaError_t e = cudaSuccess;
+            plan.copies(k + 1, [&](int64_t first, int64_t n, int64_t place) {
+                if (e == cudaSuccess)
+                    e = cudaMemcpyAsync(half(k + 1) + place, src + first, n * sizeof(S), cudaMemcpyDeviceToHost,
+                                        ctx->stream);
+            });
+            CU(e);
             CU(cudaEventRecord(ctx->landed[(k + 1) & 1], ctx->stream));
         }
         if (k < 0)
             continue;
         CU(cudaEventSynchronize(ctx->landed[k & 1]));
-        const S *h = half(k);
-        for (int64_t at = k * chunk, end = std::min(total, at + chunk); at < end;)
-        {
-            const int64_t q = at / per, stop = std::min(end, (q + 1) * per);
-            if (double *d = dst[q])
-                copy_out(h, stop - at, d + (at - q * per));
-            h += stop - at;
-            at = stop;
-        }
+        plan.parts(k, [&](int q, int64_t e, int64_t n, int64_t place) { copy_out(half(k) + place, n, dst[q] + e); });
     }
+    if (plan.chunks() == 0) // nothing wanted: still not before the stream's work is done
+        CU(cudaStreamSynchronize(ctx->stream));
     bounce.landed = true;
     return GRLBM_OK;
 }
