@@ -407,6 +407,8 @@ struct Step64Args
 // The fixed streaming types' step with one patch per block (step_block.cuh):
 // a block's tile is kBlockStepWarps rows of 8 or 4 cells, one per warp.
 constexpr int kBlockStepWarps = 8;
+// blocks that a grid holds along y
+constexpr int kMaxGridY = 65535;
 struct BlockStep
 {
     int run;                 // cells of a row a warp takes: a tile is `run` x kBlockStepWarps cells

@@ -8,6 +8,8 @@
 #include <cudaTypedefs.h>
 
 #include "approx_math.hpp"
+#include <algorithm>
+
 #include "device_common.cuh"
 #include "tma_util.cuh"
 
@@ -771,9 +773,15 @@ void launch_step_prec_adaptive(const PrecStepArgs &a, const DirTable &dt, bool c
     if (curved)
     {
         const size_t smem = apatch_smem(a.nd, a.ng, a.nf);
-        const dim3 tiles(nblk(a.g.nx_, kAPatchX), nblk(rows, kAPatchY));
-        if (smem <= kAPatchMaxSmem && tiles.x * tiles.y >= kAPatchMinTiles)
-            k_stream_prec_adaptive_curved<<<tiles, kAPatchThreads, smem, s>>>(a);
+        const unsigned tiles_x = nblk(a.g.nx_, kAPatchX), tiles_y = nblk(rows, kAPatchY);
+        if (smem <= kAPatchMaxSmem && tiles_x * tiles_y >= kAPatchMinTiles)
+            for (unsigned first = 0; first < tiles_y; first += kMaxGridY) // (the grid's y holds so many)
+            {
+                PrecStepArgs part = a;
+                part.g.jlo += (int64_t)first * kAPatchY;
+                k_stream_prec_adaptive_curved<<<dim3(tiles_x, std::min(tiles_y - first, (unsigned)kMaxGridY)),
+                                                kAPatchThreads, smem, s>>>(part);
+            }
         else
         {
             const dim3 sgrid(nblk(a.nd, kADirs) * (unsigned)rows, tx);

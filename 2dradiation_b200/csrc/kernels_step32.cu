@@ -1206,11 +1206,7 @@ cudaError_t block_occupancy32(bool curved, int run, int smem, int *blocks)
 
 void launch_step_block32(const Step32Args &a, const BlockStep &b, const DirTable *dt, bool curved, cudaStream_t s)
 {
-    if (b.tiles_x <= 0 || b.tiles_y <= 0)
-        return;
-    void *args[] = {const_cast<Step32Args *>(&a), const_cast<BlockStep *>(&b), &dt};
-    cudaLaunchKernel(block_kernel32(curved, b.run), dim3(b.tiles_x, b.tiles_y), dim3(block::kThreads), args,
-                     (size_t)b.smem, s);
+    block::launch_tiles(block_kernel32(curved, b.run), a, b, dt, s);
 }
 
 void launch_step_batch32(const Batch32Item *items, const int *first_tile, int n_items, int total_tiles, int flip,

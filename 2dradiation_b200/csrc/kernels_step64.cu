@@ -863,11 +863,7 @@ cudaError_t block_occupancy64(bool curved, int run, int smem, int *blocks)
 
 void launch_step_block64(const Step64Args &a, const BlockStep &b, const DirTable64 *dt, bool curved, cudaStream_t s)
 {
-    if (b.tiles_x <= 0 || b.tiles_y <= 0)
-        return;
-    void *args[] = {const_cast<Step64Args *>(&a), const_cast<BlockStep *>(&b), &dt};
-    cudaLaunchKernel(block_kernel64(curved, b.run), dim3(b.tiles_x, b.tiles_y), dim3(block::kThreads), args,
-                     (size_t)b.smem, s);
+    block::launch_tiles(block_kernel64(curved, b.run), a, b, dt, s);
 }
 
 void launch_step64(const Step64Args &a, const DirTable64 *dt, bool curved, int P, int blocks, cudaStream_t s)

@@ -33,6 +33,7 @@
 // taps and weights kept for the next cell where the window and corner stay (91
 // us: fewer reads, as many instructions).
 #pragma once
+#include <algorithm>
 #include <type_traits>
 
 #include "device_common.cuh"
@@ -403,6 +404,21 @@ __global__ void __launch_bounds__(kThreads, F::kMinBlocks)
                 atomicMax(a.iter_max, atomicMax(stat + 1, 0u));
             }
         }
+    }
+}
+
+// Launches the kernel over the step's tiles: rows of tiles lie along the
+// grid's y, as many at a time as that may hold.
+template <class Args, class Table>
+void launch_tiles(const void *kernel, const Args &a, const BlockStep &b, const Table *dt, cudaStream_t s)
+{
+    for (int first = 0; b.tiles_x > 0 && first < b.tiles_y; first += kMaxGridY)
+    {
+        Args part = a;
+        part.g.jlo += (int64_t)first * kBlockStepWarps;
+        void *args[] = {&part, const_cast<BlockStep *>(&b), &dt};
+        cudaLaunchKernel(kernel, dim3(b.tiles_x, std::min(b.tiles_y - first, kMaxGridY)), dim3(kThreads), args,
+                         (size_t)b.smem, s);
     }
 }
 
