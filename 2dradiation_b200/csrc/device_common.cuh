@@ -413,6 +413,8 @@ struct BlockStep
 {
     int run;                 // cells of a row a warp takes: a tile is `run` x kBlockStepWarps cells
     int tiles_x, tiles_y;    // tiles over the slab rows
+    int resident;            // blocks the GPU holds at once
+    int grid;                // blocks that share the tiles (0, or no fewer than the tiles: one each)
     int ss;                  // row stride of the streamed values
     int q, nd4;              // row types; directions rounded up to 4
     int parts;               // lanes that share a run's cells of one direction (flat streaming)

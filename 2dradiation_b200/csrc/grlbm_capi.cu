@@ -641,6 +641,7 @@ int set_block_step(grlbm_ctx *ctx)
     for (int k = 0; k < 2; k++)
     {
         ctx->blk[k] = b[pick];
+        ctx->blk[k].resident = per_sm[pick] * sms;
         const cudaError_t e = ctx->fast64 ? encode_state_map64(&ctx->blk[k].map, ctx->I[k].as<double>(), ctx->geo.nx,
                                                                ctx->geo.ny, dp, b[pick].run, kBlockStepWarps)
                                           : encode_state_map32(&ctx->blk[k].map, ctx->I[k].as<float>(), ctx->geo.nx,
@@ -651,10 +652,12 @@ int set_block_step(grlbm_ctx *ctx)
     return GRLBM_OK;
 }
 
-// The block step's tiles over the rows of the context's band.
-BlockStep block_step(const grlbm_ctx *ctx, int from)
+// The block step's tiles over the rows of the context's band, on a grid of
+// `blocks` (0: one a tile).
+BlockStep block_step(const grlbm_ctx *ctx, int from, int blocks)
 {
     BlockStep b = ctx->blk[from];
+    b.grid = blocks;
     const int64_t rows = ctx->gd.jhi - ctx->gd.jlo;
     b.tiles_x = (int)((ctx->gd.nx_ + b.run - 1) / b.run);
     b.tiles_y = rows <= 0 ? 0 : (int)((rows + kBlockStepWarps - 1) / kBlockStepWarps);
@@ -782,12 +785,11 @@ int check_tables(grlbm_ctx *ctx)
 // Enqueue one step starting from buffer `from` (no sync).
 // (sources: LoadInitialData at the top of the step; off for the second and
 // later row ranges of a step enqueued in parts.  blocks: the tiled forms'
-// grid, 0 for the context's own)
+// grid, 0 for the step's own)
 int enqueue_step(grlbm_ctx *ctx, int from, bool sources = true, int blocks = 0)
 {
     const bool curved = is_curved(ctx);
-    if (blocks <= 0)
-        blocks = ctx->step_blocks;
+    const int tile_blocks = blocks > 0 ? blocks : ctx->step_blocks; // the warp-per-tile kernels'
     unsigned long long *cnt = ctx->counters.as<unsigned long long>();
     if (ctx->fast64)
     {
@@ -795,11 +797,11 @@ int enqueue_step(grlbm_ctx *ctx, int from, bool sources = true, int blocks = 0)
             launch_sources64L(ctx->I[from].as<double>(), ctx->sl, ctx->st.n, ctx->src_nodes.as<int64_t>(),
                               ctx->src_vals.as<double>(), ctx->nsrc, ctx->stream);
         if (ctx->blk[from].smem)
-            launch_step_block64(step64_args(ctx, from), block_step(ctx, from), ctx->dirs64t.as<DirTable64>(), curved,
+            launch_step_block64(step64_args(ctx, from), block_step(ctx, from, blocks), ctx->dirs64t.as<DirTable64>(), curved,
                                 ctx->stream);
         else
-            launch_step64(step64_args(ctx, from), ctx->dirs64t.as<DirTable64>(), curved, ctx->passes, blocks,
-                          ctx->stream);
+            launch_step64(step64_args(ctx, from), ctx->dirs64t.as<DirTable64>(), curved, ctx->passes,
+                          tile_blocks, ctx->stream);
     }
     else if (ctx->fp32)
     {
@@ -807,10 +809,10 @@ int enqueue_step(grlbm_ctx *ctx, int from, bool sources = true, int blocks = 0)
             launch_sources32(ctx->I[from].as<float>(), ctx->sl, ctx->st.n, ctx->src_nodes.as<int64_t>(),
                              ctx->src_vals.as<float>(), ctx->nsrc, ctx->stream);
         if (ctx->blk[from].smem)
-            launch_step_block32(step32_args(ctx, from), block_step(ctx, from), ctx->dirs32t.as<DirTable>(), curved,
+            launch_step_block32(step32_args(ctx, from), block_step(ctx, from, blocks), ctx->dirs32t.as<DirTable>(), curved,
                                 ctx->stream);
         else if (!is_adaptive(ctx))
-            launch_step32(step32_args(ctx, from), ctx->dirs, curved, ctx->passes, blocks, ctx->stream);
+            launch_step32(step32_args(ctx, from), ctx->dirs, curved, ctx->passes, tile_blocks, ctx->stream);
         else
         {
             PrecStepArgs a = prec_args(ctx, from);
@@ -2606,10 +2608,10 @@ int batch_build(grlbm_batch *b)
         first[k + 1] += step32_tiles(c);
     }
     b->total_tiles = first[n];
-    // the concurrent shapes' grids: each problem's own persistent grid, or
-    // (blocks_per_sm = -m) its share of m GPUs' worth of resident blocks by
-    // its estimated cost, so that the problems' kernels are resident side by
-    // side instead of each filling the GPU in turn
+    // the concurrent shapes' grids: each problem's own (0), or (blocks_per_sm
+    // = -m) its share of m GPUs' worth of resident blocks by its estimated
+    // cost, so that the problems' kernels are resident side by side instead of
+    // each filling the GPU in turn
     b->grid.assign(n, 0);
     double wsum = 0.0;
     for (int k = 0; k < n; k++)
@@ -2617,10 +2619,9 @@ int batch_build(grlbm_batch *b)
     for (int k = 0; k < n; k++)
     {
         const grlbm_ctx *c = b->ctx[order[k]];
-        b->grid[k] = c->step_blocks;
+        const int own = c->blk[0].smem ? c->blk[0].resident : c->step_blocks;
         if (b->blocks_per_sm < 0 && is_tiled(c)) // the other forms' grids cover their work once
-            b->grid[k] = std::max(1, std::min(c->step_blocks, (int)std::ceil(-b->blocks_per_sm * c->step_blocks *
-                                                                             batch_cost(c) / wsum)));
+            b->grid[k] = std::max(1, std::min(own, (int)std::ceil(-b->blocks_per_sm * own * batch_cost(c) / wsum)));
     }
     if (alloc(nullptr, b->d_items, n * sizeof(Batch32Item)) || alloc(nullptr, b->d_first, (n + 1) * sizeof(int)))
         return bfail(b, GRLBM_ERR_CUDA, "cannot allocate the batch launch list");

@@ -1099,7 +1099,7 @@ int step32_batch_item_bytes(int q) { return (int)((sizeof(Step32Args) + sizeof(D
 
 size_t step32_batch_smem(int warp_stride) { return (size_t)kRowtabOffset + 128 + (size_t)kWarps * warp_stride; }
 
-static const void *block_kernel32(bool curved, int run);
+static const void *block_kernel32(bool curved, int run, bool share);
 
 cudaError_t prepare_step32()
 {
@@ -1119,8 +1119,8 @@ cudaError_t prepare_step32()
     GRLBM_PREP(8)
 #undef GRLBM_PREP
     for (int run = 4; run <= 8; run += 4)
-        for (int curved = 0; curved < 2 && e == cudaSuccess; curved++)
-            e = cudaFuncSetAttribute(block_kernel32(curved != 0, run), cudaFuncAttributeMaxDynamicSharedMemorySize,
+        for (int k = 0; k < 4 && e == cudaSuccess; k++)
+            e = cudaFuncSetAttribute(block_kernel32(k & 1, run, k & 2), cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      kStep32MaxSmem);
     if (e == cudaSuccess)
         e = set_smem_limit<true, 1, true>();
@@ -1190,23 +1190,28 @@ void block_layout32(BlockStep &b, int nd, int dp, int q, bool curved)
     block::set_layout<Form32>(b, nd, step32_patch_node_floats(dp), q, curved, Form32::flat_bytes(nd, b.run));
 }
 
-static const void *block_kernel32(bool curved, int run)
+template <bool CURVED>
+static const void *block_kernel32(int run, bool share)
 {
-    if (run == 4)
-        return curved ? (const void *)block::k_step_block<Form32, true, 4>
-                      : (const void *)block::k_step_block<Form32, false, 4>;
-    return curved ? (const void *)block::k_step_block<Form32, true, 8>
-                  : (const void *)block::k_step_block<Form32, false, 8>;
+    if (share)
+        return run == 4 ? (const void *)block::k_step_block<Form32, CURVED, 4, true>
+                        : (const void *)block::k_step_block<Form32, CURVED, 8, true>;
+    return run == 4 ? (const void *)block::k_step_block<Form32, CURVED, 4, false>
+                    : (const void *)block::k_step_block<Form32, CURVED, 8, false>;
+}
+static const void *block_kernel32(bool curved, int run, bool share)
+{
+    return curved ? block_kernel32<true>(run, share) : block_kernel32<false>(run, share);
 }
 
 cudaError_t block_occupancy32(bool curved, int run, int smem, int *blocks)
 {
-    return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks, block_kernel32(curved, run), block::kThreads, smem);
+    return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks, block_kernel32(curved, run, false), block::kThreads, smem);
 }
 
 void launch_step_block32(const Step32Args &a, const BlockStep &b, const DirTable *dt, bool curved, cudaStream_t s)
 {
-    block::launch_tiles(block_kernel32(curved, b.run), a, b, dt, s);
+    block::launch_tiles(block_kernel32(curved, b.run, false), block_kernel32(curved, b.run, true), a, b, dt, s);
 }
 
 void launch_step_batch32(const Batch32Item *items, const int *first_tile, int n_items, int total_tiles, int flip,

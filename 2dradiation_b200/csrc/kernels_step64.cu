@@ -798,7 +798,7 @@ size_t step64_smem(int tx, int ty, int dp, int nd, int q)
            (size_t)kWarps * (size_t)step64_warp_stride(tx, ty, dp, nd);
 }
 
-static const void *block_kernel64(bool curved, int run);
+static const void *block_kernel64(bool curved, int run, bool share);
 
 cudaError_t prepare_step64()
 {
@@ -818,8 +818,8 @@ cudaError_t prepare_step64()
     GRLBM_PREP(8)
 #undef GRLBM_PREP
     for (int run = 4; run <= 8; run += 4)
-        for (int curved = 0; curved < 2 && e == cudaSuccess; curved++)
-            e = cudaFuncSetAttribute(block_kernel64(curved != 0, run), cudaFuncAttributeMaxDynamicSharedMemorySize,
+        for (int k = 0; k < 4 && e == cudaSuccess; k++)
+            e = cudaFuncSetAttribute(block_kernel64(k & 1, run, k & 2), cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      kStep32MaxSmem);
     return e;
 }
@@ -847,23 +847,28 @@ void block_layout64(BlockStep &b, int nd, int dp, int q, bool curved)
     block::set_layout<Form64>(b, nd, step64_patch_node_elems(dp), q, curved, Form64::flat_bytes(nd, b.run));
 }
 
-static const void *block_kernel64(bool curved, int run)
+template <bool CURVED>
+static const void *block_kernel64(int run, bool share)
 {
-    if (run == 4)
-        return curved ? (const void *)block::k_step_block<Form64, true, 4>
-                      : (const void *)block::k_step_block<Form64, false, 4>;
-    return curved ? (const void *)block::k_step_block<Form64, true, 8>
-                  : (const void *)block::k_step_block<Form64, false, 8>;
+    if (share)
+        return run == 4 ? (const void *)block::k_step_block<Form64, CURVED, 4, true>
+                        : (const void *)block::k_step_block<Form64, CURVED, 8, true>;
+    return run == 4 ? (const void *)block::k_step_block<Form64, CURVED, 4, false>
+                    : (const void *)block::k_step_block<Form64, CURVED, 8, false>;
+}
+static const void *block_kernel64(bool curved, int run, bool share)
+{
+    return curved ? block_kernel64<true>(run, share) : block_kernel64<false>(run, share);
 }
 
 cudaError_t block_occupancy64(bool curved, int run, int smem, int *blocks)
 {
-    return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks, block_kernel64(curved, run), block::kThreads, smem);
+    return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks, block_kernel64(curved, run, false), block::kThreads, smem);
 }
 
 void launch_step_block64(const Step64Args &a, const BlockStep &b, const DirTable64 *dt, bool curved, cudaStream_t s)
 {
-    block::launch_tiles(block_kernel64(curved, b.run), a, b, dt, s);
+    block::launch_tiles(block_kernel64(curved, b.run, false), block_kernel64(curved, b.run, true), a, b, dt, s);
 }
 
 void launch_step64(const Step64Args &a, const DirTable64 *dt, bool curved, int P, int blocks, cudaStream_t s)

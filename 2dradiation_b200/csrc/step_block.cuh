@@ -80,7 +80,10 @@ __device__ __forceinline__ void store_row(T *p, const T (&v)[V])
 // curved, far_curved, flat_tables and flat (one streamed value), moments (a
 // lane's three sums), coeffs (the collide map's) and changing (whether the
 // iteration goes on).
-template <class F, bool CURVED, int RUN>
+// SHARE: the grid is cut to a share of the GPU (a batch's launch shapes below
+// 0): a block takes every gridDim.x-th tile, copies the tables once, and
+// stages its next patch as soon as all of its warps have streamed theirs.
+template <class F, bool CURVED, int RUN, bool SHARE>
 __global__ void __launch_bounds__(kThreads, F::kMinBlocks)
     k_step_block(const __grid_constant__ typename F::Args a, const __grid_constant__ BlockStep b,
                  const typename F::Table *__restrict__ dtp)
@@ -102,289 +105,312 @@ __global__ void __launch_bounds__(kThreads, F::kMinBlocks)
     T4 *map = reinterpret_cast<T4 *>(smem + b.off_map) + warp * RUN; // phase 3's map of each cell
     unsigned *stat = reinterpret_cast<unsigned *>(smem + 16);             // cycles, most cycles, warps done
     const unsigned bar = smem_addr(smem);
-    const int x0 = (int)blockIdx.x * RUN, y0 = (int)a.g.jlo - 1 + (int)blockIdx.y * kBlockStepWarps;
+    auto stage = [&](int x, int y) { // (thread 0)
+        mbar_arrive_expect(bar, (unsigned)(px * (kBlockStepWarps + 2) * dps * (int)sizeof(T)));
+        tma_load_4d(smem_addr(patch), &b.map, 0, 0, x, y, bar);
+    };
+    int tile = (int)blockIdx.x; // SHARE: row after row
+    int x0 = (SHARE ? tile % b.tiles_x : tile) * RUN;
+    int y0 = (int)a.g.jlo - 1 + (SHARE ? tile / b.tiles_x : (int)blockIdx.y) * kBlockStepWarps;
     if (threadIdx.x == 0)
     {
         mbar_init(bar, 1);
-        mbar_arrive_expect(bar, (unsigned)(px * (kBlockStepWarps + 2) * dps * (int)sizeof(T)));
-        tma_load_4d(smem_addr(patch), &b.map, 0, 0, x0, y0, bar);
+        stage(x0, y0);
         stat[0] = stat[1] = stat[2] = 0u;
     }
-    // the warp's run: cells (xw + c, yw), c < ncells, of the interior
-    // (lanes of a cell: h, e; with runs of 4 the upper lanes idle in phase 2)
-    const int c = lane & 7, h = (lane >> 3) & 1, e = lane >> 4;
-    const int xw = x0, yw = y0 + warp;
-    const int ncells = yw < (int)a.g.jhi - 1 ? max(0, min(RUN, nx_ - xw)) : 0;
-    const int total = ncells * nd;
-    const bool cact = c < ncells;
-    const int cij = (1 + xw + (cact ? c : 0)) + (1 + (ncells ? yw : y0)) * nxn;
-    const int cfl = cact ? (int)a.flags[cij] : 3;
-    const typename F::Rec *rp = nullptr;
-    typename F::Rec r[2];
-    if (CURVED)
+    unsigned it_sum = 0u, it_max = 0u, parity = 0u;
+    for (bool first = true;; first = false)
     {
-        rp = a.rec + ((size_t)(xw + yw * nx_) * (size_t)nd + (size_t)lane);
-#pragma unroll
-        for (int k = 0; k < 2; k++)
-            r[k] = F::load(rp + 32 * k, lane + 32 * k < total);
-        for (int k = threadIdx.x; k < b.q * 12; k += kThreads)
+        // the warp's run: cells (xw + c, yw), c < ncells, of the interior
+        // (lanes of a cell: h, e; with runs of 4 the upper lanes idle in phase 2)
+        const int c = lane & 7, h = (lane >> 3) & 1, e = lane >> 4;
+        const int xw = x0, yw = y0 + warp;
+        const int ncells = yw < (int)a.g.jhi - 1 ? max(0, min(RUN, nx_ - xw)) : 0;
+        const int total = ncells * nd;
+        const bool cact = c < ncells;
+        const int cij = (1 + xw + (cact ? c : 0)) + (1 + (ncells ? yw : y0)) * nxn;
+        const int cfl = cact ? (int)a.flags[cij] : 3;
+        const typename F::Rec *rp = nullptr;
+        typename F::Rec r[2];
+        const bool tables = !SHARE || first;
+        if (CURVED)
         {
-            const int row = k / 12, col = k - 12 * row;
-            if (col < F::kRow)
-                rowtab[row * F::kRow + col] = __ldg(dtp->rowtab + k);
-        }
-    }
-    for (int k = threadIdx.x; k < nd; k += kThreads)
-    {
-        const T *cf = dtp->dirc + 8 * k;
-        T *m = momtab + 8 * k;
-        m[0] = cf[0], m[1] = cf[1], m[2] = cf[2], m[3] = cf[6];
-        m[4] = cf[3], m[5] = cf[4], m[6] = cf[5], m[7] = cf[7];
-        n1s[k] = cf[6], n2s[k] = cf[7];
-    }
-    if (threadIdx.x < 18)
-        wmom[threadIdx.x] = __ldg(dtp->wmom + threadIdx.x);
-    if (!CURVED)
-        F::flat_tables(a, b, *dtp, smem + b.off_flat, x0, y0);
-    __syncthreads();
-    unsigned parity = 0;
-    if (!step::wait_tile(bar, parity, a.fault))
-        return;
-
-    // ---- phase 1: stream ----
-    const unsigned holes = __ballot_sync(0xffffffffu, lane < 8 && cact && (cfl & 2)); // cells that stream zeros
-    const T *wpatch = patch + warp * px * dps;
-    const int pdp = px * dps;
-    if (CURVED)
-    {
-        // the run's (cell, direction) pairs in order, 32 at a time
-        int cell = 0, d = lane;
-        while (d >= nd)
-            d -= nd, cell++;
-        for (int e0 = 0; e0 < total; e0 += 64)
-        {
-            typename F::Rec n[2];
+            rp = a.rec + ((size_t)(xw + yw * nx_) * (size_t)nd + (size_t)lane);
 #pragma unroll
             for (int k = 0; k < 2; k++)
-                n[k] = F::load(rp + (e0 + 64 + 32 * k), e0 + 64 + 32 * k + lane < total);
-#pragma unroll
-            for (int k = 0; k < 2; k++)
+                r[k] = F::load(rp + 32 * k, lane + 32 * k < total);
+            for (int k = tables ? threadIdx.x : b.q * 12; k < b.q * 12; k += kThreads)
             {
-                if (e0 + 32 * k + lane < total)
-                {
-                    bool far;
-                    T v = F::curved(r[k], wpatch + cell * dps, dps, pdp, rowtab, far);
-                    if ((holes >> cell) & 1u)
-                        v = T(0);
-                    else if (far)
-                        v = F::far_curved(a, *dtp, xw + 1 + cell, yw + 1, xw + cell + yw * nx_, d);
-                    S[cell * ss + d] = v;
-                }
-                d += 32;
-                while (d >= nd)
-                    d -= nd, cell++;
-                r[k] = n[k];
+                const int row = k / 12, col = k - 12 * row;
+                if (col < F::kRow)
+                    rowtab[row * F::kRow + col] = __ldg(dtp->rowtab + k);
             }
         }
-    }
-    else
-    {
-        // a lane takes one direction through `span` cells of the run: a cell's
-        // right-hand nodes are the next one's left-hand ones
-        const int ncols = nd * b.parts, span = RUN / b.parts;
-        for (int p0 = 0; p0 < ncols; p0 += 32)
+        for (int k = tables ? threadIdx.x : nd; k < nd; k += kThreads)
         {
-            int d = p0 + lane, first = 0;
+            const T *cf = dtp->dirc + 8 * k;
+            T *m = momtab + 8 * k;
+            m[0] = cf[0], m[1] = cf[1], m[2] = cf[2], m[3] = cf[6];
+            m[4] = cf[3], m[5] = cf[4], m[6] = cf[5], m[7] = cf[7];
+            n1s[k] = cf[6], n2s[k] = cf[7];
+        }
+        if (tables && threadIdx.x < 18)
+            wmom[threadIdx.x] = __ldg(dtp->wmom + threadIdx.x);
+        if (!CURVED)
+            F::flat_tables(a, b, *dtp, smem + b.off_flat, x0, y0);
+        __syncthreads();
+        if (!step::wait_tile(bar, parity, a.fault))
+            return;
+
+        // ---- phase 1: stream ----
+        const unsigned holes = __ballot_sync(0xffffffffu, lane < 8 && cact && (cfl & 2)); // cells that stream zeros
+        const T *wpatch = patch + warp * px * dps;
+        const int pdp = px * dps;
+        if (CURVED)
+        {
+            // the run's (cell, direction) pairs in order, 32 at a time
+            int cell = 0, d = lane;
             while (d >= nd)
-                d -= nd, first += span;
-            const int n = min(span, ncells - first);
-            if (p0 + lane < ncols && n > 0)
-                F::flat_run(a, b, *dtp, smem + b.off_flat, wpatch + first * dps, S + first * ss + d, n, dps, pdp, ss,
-                            first, warp, xw + 1 + first, yw + 1, d);
-        }
-    }
-    __syncwarp();
-
-    // ---- phase 2: moments and collide, four lanes per cell ----
-    unsigned it_sum = 0u, it_max = 0u;
-    if (cact)
-    {
-        const unsigned quad = 0x01010101u << c; // the cell's lanes
-        const T u1 = __ldg(a.u1 + cij), u2 = __ldg(a.u2 + cij), lor = __ldg(a.lor + cij);
-        const T adt = __ldg(a.adt + cij), eta = __ldg(a.eta + cij), k0 = __ldg(a.k0 + cij);
-        const T k3 = __ldg(a.k3 + cij), kak0 = __ldg(a.ka + cij) + k0;
-        const T scale = CURVED ? __ldg(a.ia3 + cij) : T(1);
-        T *Sc = S + c * ss;
-        T m[6];
-        {
-            T own[3];
-            F::moments(Sc, momtab + 4 * e, nd, h, quad, own);
-#pragma unroll
-            for (int q = 0; q < 3; q++)
+                d -= nd, cell++;
+            for (int e0 = 0; e0 < total; e0 += 64)
             {
-                const T other = __shfl_xor_sync(quad, own[q], 16);
-                m[q] = e ? other : own[q];
-                m[3 + q] = e ? own[q] : other;
-            }
-        }
-        T og = T(1), oa = T(0), ob1 = T(0), ob2 = T(0);
-        if (!(cfl & 1))
-        {
-            int cycles = 0;
-            const bool rest = (u1 == T(0)) && (u2 == T(0));
-            // m_new[q] = A[q] + (eta + k0 fE) B[q] + k3 (fFx C[q] + fFy D[q])
-            T A6[6], B6[6], C6[6], D6[6];
-            T g0 = T(0), h0 = T(0);
-            if (rest)
-            {
-                g0 = T(1) / (T(1) + adt * kak0);
-                h0 = adt * g0;
+                typename F::Rec n[2];
 #pragma unroll
-                for (int q = 0; q < 6; q++)
+                for (int k = 0; k < 2; k++)
+                    n[k] = F::load(rp + (e0 + 64 + 32 * k), e0 + 64 + 32 * k + lane < total);
+#pragma unroll
+                for (int k = 0; k < 2; k++)
                 {
-                    A6[q] = g0 * m[q];
-                    B6[q] = h0 * wmom[q];
-                    C6[q] = h0 * wmom[6 + q];
-                    D6[q] = h0 * wmom[12 + q];
+                    if (e0 + 32 * k + lane < total)
+                    {
+                        bool far;
+                        T v = F::curved(r[k], wpatch + cell * dps, dps, pdp, rowtab, far);
+                        if ((holes >> cell) & 1u)
+                            v = T(0);
+                        else if (far)
+                            v = F::far_curved(a, *dtp, xw + 1 + cell, yw + 1, xw + cell + yw * nx_, d);
+                        S[cell * ss + d] = v;
+                    }
+                    d += 32;
+                    while (d >= nd)
+                        d -= nd, cell++;
+                    r[k] = n[k];
                 }
             }
-            else
-            {
-                // lane e = 0 sums A and B, lane e = 1 C and D; each computes the
-                // map's coefficients of every second of the directions of its
-                // parity h and hands the other lane's share over
-                T X6[6], Y6[6];
-#pragma unroll
-                for (int q = 0; q < 6; q++)
-                    X6[q] = Y6[q] = T(0);
-                const unsigned pair = 0x00010001u << (lane & 15); // both lanes of this parity
-                for (int d0 = h; d0 < nd; d0 += 4)
-                {
-                    const int dd = min(d0 + 2 * e, nd - 1);
-                    const T w = momtab[8 * dd];
-                    T g, hh, q1, q2;
-                    F::coeffs(n1s[dd], n2s[dd], u1, u2, lor, adt, kak0, g, hh, q1, q2);
-                    const T gs = w * g * Sc[dd], wh = w * hh;
-                    const T whq1 = wh * q1, whq2 = wh * q2;
-                    const T ox = __shfl_xor_sync(pair, e ? gs : whq1, 16), oy = __shfl_xor_sync(pair, e ? wh : whq2, 16);
-                    const T x[2] = {e ? ox : gs, e ? whq1 : ox}, y[2] = {e ? oy : wh, e ? whq2 : oy};
-#pragma unroll
-                    for (int s = 0; s < 2; s++)
-                        if (d0 + 2 * s < nd)
-                        {
-                            const T n1 = n1s[d0 + 2 * s], n2 = n2s[d0 + 2 * s];
-                            const T mu[6] = {T(1), n1, n2, n1 * n1, n1 * n2, n2 * n2};
-#pragma unroll
-                            for (int q = 0; q < 6; q++)
-                            {
-                                X6[q] = F::fma(x[s], mu[q], X6[q]);
-                                Y6[q] = F::fma(y[s], mu[q], Y6[q]);
-                            }
-                        }
-                }
-#pragma unroll
-                for (int q = 0; q < 6; q++)
-                {
-                    X6[q] += __shfl_xor_sync(quad, X6[q], 8);
-                    Y6[q] += __shfl_xor_sync(quad, Y6[q], 8);
-                    const T ox = __shfl_xor_sync(quad, X6[q], 16), oy = __shfl_xor_sync(quad, Y6[q], 16);
-                    A6[q] = e ? ox : X6[q], B6[q] = e ? oy : Y6[q];
-                    C6[q] = e ? X6[q] : ox, D6[q] = e ? Y6[q] : oy;
-                }
-            }
-            bool changing = true;
-            T fE = T(0), fFx = T(0), fFy = T(0);
-            while (changing && cycles < 100)
-            {
-                cycles++;
-                const T pE = m[0], pFx = m[1], pFy = m[2], pPxx = m[3], pPxy = m[4], pPyy = m[5];
-                const T uF = u1 * pFx + u2 * pFy;
-                const T uxP = u1 * pPxx + u2 * pPxy;
-                const T uyP = u1 * pPxy + u2 * pPyy;
-                const T uuP = u1 * uxP + u2 * uyP;
-                fE = lor * lor * (pE - T(2) * uF + uuP);
-                const T rr = lor / (T(1) + lor) * ((T(2) * lor + T(1)) * uF - lor * uuP);
-                fFx = lor * lor * (pFx - lor * pE * u1 - uxP + u1 * rr);
-                fFy = lor * lor * (pFy - lor * pE * u2 - uyP + u2 * rr);
-                const T ee = eta + k0 * fE;
-                const T prev[6] = {pE, pFx, pFy, pPxx, pPxy, pPyy};
-#pragma unroll
-                for (int q = 0; q < 6; q++)
-                    m[q] = A6[q] + ee * B6[q] + k3 * (fFx * C6[q] + fFy * D6[q]);
-                changing = F::changing(prev, m);
-            }
-            // the intensities of the last iterate: at rest the affine map phase
-            // 3 applies; a moving fluid's here, every fourth direction a lane
-            const T ee = eta + k0 * fE;
-            if (rest)
-            {
-                og = g0 * scale;
-                oa = h0 * ee * scale;
-                ob1 = h0 * k3 * fFx * scale;
-                ob2 = h0 * k3 * fFy * scale;
-            }
-            else
-            {
-                for (int dd = h + 2 * e; dd < nd; dd += 4)
-                {
-                    T g, hh, q1, q2;
-                    F::coeffs(n1s[dd], n2s[dd], u1, u2, lor, adt, kak0, g, hh, q1, q2);
-                    Sc[dd] = (g * Sc[dd] + hh * (ee + k3 * (q1 * fFx + q2 * fFy))) * scale;
-                }
-            }
-            if (lane < 8)
-                it_sum = it_max = (unsigned)cycles;
         }
         else
-            og = scale;
-        if (h == 0)
-#pragma unroll
-            for (int q = 0; q < 3; q++)
-                a.mom[(size_t)cij + (size_t)(3 * e + q) * (size_t)a.g.nxy] = e ? m[3 + q] : m[q];
-        if (lane < 8)
         {
-            T4 o;
-            o.x = og, o.y = oa, o.z = ob1, o.w = ob2;
-            map[c] = o;
+            // a lane takes one direction through `span` cells of the run: a cell's
+            // right-hand nodes are the next one's left-hand ones
+            const int ncols = nd * b.parts, span = RUN / b.parts;
+            for (int p0 = 0; p0 < ncols; p0 += 32)
+            {
+                int d = p0 + lane, from = 0;
+                while (d >= nd)
+                    d -= nd, from += span;
+                const int n = min(span, ncells - from);
+                if (p0 + lane < ncols && n > 0)
+                    F::flat_run(a, b, *dtp, smem + b.off_flat, wpatch + from * dps, S + from * ss + d, n, dps, pdp, ss,
+                                from, warp, xw + 1 + from, yw + 1, d);
+            }
         }
-    }
-    __syncwarp();
-
-    // ---- phase 3: the run's new state, and the mirrored directions 0..3
-    // after each cell's last one ----
-    T *out = a.Iout + (size_t)(1 + xw + (1 + yw) * nxn) * (size_t)dp;
-    // V directions a lane
-    auto store = [&](auto vc) {
-        constexpr int V = decltype(vc)::value;
-        const int nv = nd / V;
-        int k = lane, cl = 0;
-        while (k >= nv)
-            k -= nv, cl++;
-        while (cl < ncells)
+        if (SHARE)
         {
-            const T4 o = map[cl];
-            T v[V], n1[V], n2[V];
-            load_row<V>(v, S + cl * ss + V * k);
-            load_row<V>(n1, n1s + V * k);
-            load_row<V>(n2, n2s + V * k);
+            __syncthreads();
+            tile += (int)gridDim.x;
+            x0 = tile % b.tiles_x * RUN;
+            y0 = (int)a.g.jlo - 1 + tile / b.tiles_x * kBlockStepWarps;
+            if (threadIdx.x == 0 && tile < b.tiles_x * b.tiles_y)
+                stage(x0, y0);
+        }
+        else
+            __syncwarp();
+
+        // ---- phase 2: moments and collide, four lanes per cell ----
+        if (cact)
+        {
+            const unsigned quad = 0x01010101u << c; // the cell's lanes
+            const T u1 = __ldg(a.u1 + cij), u2 = __ldg(a.u2 + cij), lor = __ldg(a.lor + cij);
+            const T adt = __ldg(a.adt + cij), eta = __ldg(a.eta + cij), k0 = __ldg(a.k0 + cij);
+            const T k3 = __ldg(a.k3 + cij), kak0 = __ldg(a.ka + cij) + k0;
+            const T scale = CURVED ? __ldg(a.ia3 + cij) : T(1);
+            T *Sc = S + c * ss;
+            T m[6];
+            {
+                T own[3];
+                F::moments(Sc, momtab + 4 * e, nd, h, quad, own);
 #pragma unroll
-            for (int s = 0; s < V; s++)
-                v[s] = F::fma(o.x, v[s], F::fma(o.z, n1[s], F::fma(o.w, n2[s], o.y)));
-            T *p = out + cl * dp + V * k;
-            store_row<V>(p, v);
-            if (V * k < kStateMirror)
-                store_row<V>(p + nd, v);
-            k += 32;
+                for (int q = 0; q < 3; q++)
+                {
+                    const T other = __shfl_xor_sync(quad, own[q], 16);
+                    m[q] = e ? other : own[q];
+                    m[3 + q] = e ? own[q] : other;
+                }
+            }
+            T og = T(1), oa = T(0), ob1 = T(0), ob2 = T(0);
+            if (!(cfl & 1))
+            {
+                int cycles = 0;
+                const bool rest = (u1 == T(0)) && (u2 == T(0));
+                // m_new[q] = A[q] + (eta + k0 fE) B[q] + k3 (fFx C[q] + fFy D[q])
+                T A6[6], B6[6], C6[6], D6[6];
+                T g0 = T(0), h0 = T(0);
+                if (rest)
+                {
+                    g0 = T(1) / (T(1) + adt * kak0);
+                    h0 = adt * g0;
+#pragma unroll
+                    for (int q = 0; q < 6; q++)
+                    {
+                        A6[q] = g0 * m[q];
+                        B6[q] = h0 * wmom[q];
+                        C6[q] = h0 * wmom[6 + q];
+                        D6[q] = h0 * wmom[12 + q];
+                    }
+                }
+                else
+                {
+                    // lane e = 0 sums A and B, lane e = 1 C and D; each computes the
+                    // map's coefficients of every second of the directions of its
+                    // parity h and hands the other lane's share over
+                    T X6[6], Y6[6];
+#pragma unroll
+                    for (int q = 0; q < 6; q++)
+                        X6[q] = Y6[q] = T(0);
+                    const unsigned pair = 0x00010001u << (lane & 15); // both lanes of this parity
+                    for (int d0 = h; d0 < nd; d0 += 4)
+                    {
+                        const int dd = min(d0 + 2 * e, nd - 1);
+                        const T w = momtab[8 * dd];
+                        T g, hh, q1, q2;
+                        F::coeffs(n1s[dd], n2s[dd], u1, u2, lor, adt, kak0, g, hh, q1, q2);
+                        const T gs = w * g * Sc[dd], wh = w * hh;
+                        const T whq1 = wh * q1, whq2 = wh * q2;
+                        const T ox = __shfl_xor_sync(pair, e ? gs : whq1, 16), oy = __shfl_xor_sync(pair, e ? wh : whq2, 16);
+                        const T x[2] = {e ? ox : gs, e ? whq1 : ox}, y[2] = {e ? oy : wh, e ? whq2 : oy};
+#pragma unroll
+                        for (int s = 0; s < 2; s++)
+                            if (d0 + 2 * s < nd)
+                            {
+                                const T n1 = n1s[d0 + 2 * s], n2 = n2s[d0 + 2 * s];
+                                const T mu[6] = {T(1), n1, n2, n1 * n1, n1 * n2, n2 * n2};
+#pragma unroll
+                                for (int q = 0; q < 6; q++)
+                                {
+                                    X6[q] = F::fma(x[s], mu[q], X6[q]);
+                                    Y6[q] = F::fma(y[s], mu[q], Y6[q]);
+                                }
+                            }
+                    }
+#pragma unroll
+                    for (int q = 0; q < 6; q++)
+                    {
+                        X6[q] += __shfl_xor_sync(quad, X6[q], 8);
+                        Y6[q] += __shfl_xor_sync(quad, Y6[q], 8);
+                        const T ox = __shfl_xor_sync(quad, X6[q], 16), oy = __shfl_xor_sync(quad, Y6[q], 16);
+                        A6[q] = e ? ox : X6[q], B6[q] = e ? oy : Y6[q];
+                        C6[q] = e ? X6[q] : ox, D6[q] = e ? Y6[q] : oy;
+                    }
+                }
+                bool changing = true;
+                T fE = T(0), fFx = T(0), fFy = T(0);
+                while (changing && cycles < 100)
+                {
+                    cycles++;
+                    const T pE = m[0], pFx = m[1], pFy = m[2], pPxx = m[3], pPxy = m[4], pPyy = m[5];
+                    const T uF = u1 * pFx + u2 * pFy;
+                    const T uxP = u1 * pPxx + u2 * pPxy;
+                    const T uyP = u1 * pPxy + u2 * pPyy;
+                    const T uuP = u1 * uxP + u2 * uyP;
+                    fE = lor * lor * (pE - T(2) * uF + uuP);
+                    const T rr = lor / (T(1) + lor) * ((T(2) * lor + T(1)) * uF - lor * uuP);
+                    fFx = lor * lor * (pFx - lor * pE * u1 - uxP + u1 * rr);
+                    fFy = lor * lor * (pFy - lor * pE * u2 - uyP + u2 * rr);
+                    const T ee = eta + k0 * fE;
+                    const T prev[6] = {pE, pFx, pFy, pPxx, pPxy, pPyy};
+#pragma unroll
+                    for (int q = 0; q < 6; q++)
+                        m[q] = A6[q] + ee * B6[q] + k3 * (fFx * C6[q] + fFy * D6[q]);
+                    changing = F::changing(prev, m);
+                }
+                // the intensities of the last iterate: at rest the affine map phase
+                // 3 applies; a moving fluid's here, every fourth direction a lane
+                const T ee = eta + k0 * fE;
+                if (rest)
+                {
+                    og = g0 * scale;
+                    oa = h0 * ee * scale;
+                    ob1 = h0 * k3 * fFx * scale;
+                    ob2 = h0 * k3 * fFy * scale;
+                }
+                else
+                {
+                    for (int dd = h + 2 * e; dd < nd; dd += 4)
+                    {
+                        T g, hh, q1, q2;
+                        F::coeffs(n1s[dd], n2s[dd], u1, u2, lor, adt, kak0, g, hh, q1, q2);
+                        Sc[dd] = (g * Sc[dd] + hh * (ee + k3 * (q1 * fFx + q2 * fFy))) * scale;
+                    }
+                }
+                if (lane < 8)
+                {
+                    it_sum += (unsigned)cycles;
+                    it_max = max(it_max, (unsigned)cycles);
+                }
+            }
+            else
+                og = scale;
+            if (h == 0)
+#pragma unroll
+                for (int q = 0; q < 3; q++)
+                    a.mom[(size_t)cij + (size_t)(3 * e + q) * (size_t)a.g.nxy] = e ? m[3 + q] : m[q];
+            if (lane < 8)
+            {
+                T4 o;
+                o.x = og, o.y = oa, o.z = ob1, o.w = ob2;
+                map[c] = o;
+            }
+        }
+        __syncwarp();
+
+        // ---- phase 3: the run's new state, and the mirrored directions 0..3
+        // after each cell's last one ----
+        T *out = a.Iout + (size_t)(1 + xw + (1 + yw) * nxn) * (size_t)dp;
+        // V directions a lane
+        auto store = [&](auto vc) {
+            constexpr int V = decltype(vc)::value;
+            const int nv = nd / V;
+            int k = lane, cl = 0;
             while (k >= nv)
                 k -= nv, cl++;
-        }
-    };
-    if (F::kWide == 4 && (nd & 3) == 0)
-        store(std::integral_constant<int, F::kWide>{});
-    else if ((nd & 1) == 0)
-        store(std::integral_constant<int, 2>{});
-    else
-        store(std::integral_constant<int, 1>{});
+            while (cl < ncells)
+            {
+                const T4 o = map[cl];
+                T v[V], n1[V], n2[V];
+                load_row<V>(v, S + cl * ss + V * k);
+                load_row<V>(n1, n1s + V * k);
+                load_row<V>(n2, n2s + V * k);
+#pragma unroll
+                for (int s = 0; s < V; s++)
+                    v[s] = F::fma(o.x, v[s], F::fma(o.z, n1[s], F::fma(o.w, n2[s], o.y)));
+                T *p = out + cl * dp + V * k;
+                store_row<V>(p, v);
+                if (V * k < kStateMirror)
+                    store_row<V>(p + nd, v);
+                k += 32;
+                while (k >= nv)
+                    k -= nv, cl++;
+            }
+        };
+        if (F::kWide == 4 && (nd & 3) == 0)
+            store(std::integral_constant<int, F::kWide>{});
+        else if ((nd & 1) == 0)
+            store(std::integral_constant<int, 2>{});
+        else
+            store(std::integral_constant<int, 1>{});
+        if (!SHARE || tile >= b.tiles_x * b.tiles_y)
+            break;
+    }
 
     // the lambda iteration's statistics: the block's last warp adds them
     it_sum = __reduce_add_sync(0xffffffffu, it_sum);
@@ -407,11 +433,19 @@ __global__ void __launch_bounds__(kThreads, F::kMinBlocks)
     }
 }
 
-// Launches the kernel over the step's tiles: rows of tiles lie along the
-// grid's y, as many at a time as that may hold.
+// Launches the kernel over the step's tiles: `share` on a grid of b.grid
+// blocks where that is fewer than the tiles, else one block a tile: rows of
+// tiles lie along the grid's y, as many at a time as that may hold.
 template <class Args, class Table>
-void launch_tiles(const void *kernel, const Args &a, const BlockStep &b, const Table *dt, cudaStream_t s)
+void launch_tiles(const void *kernel, const void *share, const Args &a, const BlockStep &b, const Table *dt,
+                  cudaStream_t s)
 {
+    if (b.grid > 0 && b.grid < (int64_t)b.tiles_x * b.tiles_y)
+    {
+        void *args[] = {const_cast<Args *>(&a), const_cast<BlockStep *>(&b), &dt};
+        cudaLaunchKernel(share, dim3(b.grid), dim3(kThreads), args, (size_t)b.smem, s);
+        return;
+    }
     for (int first = 0; b.tiles_x > 0 && first < b.tiles_y; first += kMaxGridY)
     {
         Args part = a;
