@@ -354,11 +354,13 @@ class Radiation:
         (stream-ordered on the context's stream)."""
         self._c(lib().grlbm_copy_rows(self.h, j_first, n, C.c_void_p(buffer_ptr), 1 if to_buffer else 0))
 
-    # ---- tiles of the precision form's fixed streaming step ----
+    # ---- tiles of the FP32 and fast FP64 fixed streaming steps ----
     def set_tile_shape(self, tile_x: int, tile_y: int):
+        """A tile for the warp-per-tile step; (0, 0): the default step again."""
         self._c(lib().grlbm_set_tile_shape(self.h, tile_x, tile_y))
 
     def tile_shape(self) -> tuple:
+        """The tile in force, (0, 0) for the default step."""
         x, y = C.c_int32(), C.c_int32()
         self._c(lib().grlbm_get_tile_shape(self.h, C.byref(x), C.byref(y)))
         return (x.value, y.value)

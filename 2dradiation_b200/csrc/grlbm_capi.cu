@@ -90,7 +90,9 @@ struct grlbm_ctx
     // persistent grid, and the TMA maps of the state buffers for that tile
     int tile_x = 4, tile_y = 4, passes = 1, step_blocks = 1;
     CUtensorMap in_map[2];
-    BlockStep blk[2] = {}; // blk[k]: the one-patch-per-block step that reads buffer k (smem 0: not used)
+    BlockStep blk[2] = {}; // blk[k]: the one-patch-per-block step that reads buffer k (smem 0: it does not fit)
+    bool tile_asked = false; // a tile was asked for: the step runs the warp-per-tile kernel
+    bool tile_tuned = false; // the tile is not the default one
     cudaEvent_t landed[2] = {nullptr, nullptr}; // a half of a read-back buffer has landed
     unsigned *fault = nullptr; // mapped host word: a precision step's staging wait timed out
     int64_t ncell = 0;
@@ -565,7 +567,7 @@ int set_step32_tile(grlbm_ctx *ctx, int tx, int ty)
     ctx->tile_x = tx;
     ctx->tile_y = ty;
     ctx->step_blocks = per_sm * sms;
-    ctx->blk[0].smem = ctx->blk[1].smem = 0; // a tile asked for: the warp-per-tile kernel
+    ctx->tile_tuned = true;
     invalidate_graphs(ctx);
     return GRLBM_OK;
 }
@@ -607,7 +609,7 @@ int adaptive_departure_rows(grlbm_ctx *ctx, int32_t *rows)
 }
 
 // Sets up the one-patch-per-block step, the default where its patch fits an
-// SM (the warp-per-tile kernel runs where a tile shape is asked for, in the
+// SM (the warp-per-tile kernel runs while a tile shape is asked for, in the
 // persistent batch launch, and for the direction counts whose patch does not
 // fit).  A warp takes 8 cells of a row, or 4 where 8 would leave the GPU
 // idle: at most one tile for every second SM (64^2 x 64 directions, fast FP64:
@@ -654,6 +656,7 @@ int set_block_step(grlbm_ctx *ctx)
 
 // The block step's tiles over the rows of the context's band, on a grid of
 // `blocks` (0: one a tile).
+bool uses_block_step(const grlbm_ctx *ctx) { return ctx->blk[0].smem && !ctx->tile_asked; }
 BlockStep block_step(const grlbm_ctx *ctx, int from, int blocks)
 {
     BlockStep b = ctx->blk[from];
@@ -716,7 +719,8 @@ int default_step32_tile(grlbm_ctx *ctx)
                 continue;
         }
         const int rc = set_step32_tile(ctx, cand[best][0], cand[best][1]);
-        return rc ? rc : set_block_step(ctx);
+        ctx->tile_asked = ctx->tile_tuned = false;
+        return rc;
     }
     return GRLBM_OK;
 }
@@ -796,7 +800,7 @@ int enqueue_step(grlbm_ctx *ctx, int from, bool sources = true, int blocks = 0)
         if (sources && ctx->run.keep_source_nodes_active && ctx->nsrc > 0)
             launch_sources64L(ctx->I[from].as<double>(), ctx->sl, ctx->st.n, ctx->src_nodes.as<int64_t>(),
                               ctx->src_vals.as<double>(), ctx->nsrc, ctx->stream);
-        if (ctx->blk[from].smem)
+        if (uses_block_step(ctx))
             launch_step_block64(step64_args(ctx, from), block_step(ctx, from, blocks), ctx->dirs64t.as<DirTable64>(), curved,
                                 ctx->stream);
         else
@@ -808,7 +812,7 @@ int enqueue_step(grlbm_ctx *ctx, int from, bool sources = true, int blocks = 0)
         if (sources && ctx->run.keep_source_nodes_active && ctx->nsrc > 0)
             launch_sources32(ctx->I[from].as<float>(), ctx->sl, ctx->st.n, ctx->src_nodes.as<int64_t>(),
                              ctx->src_vals.as<float>(), ctx->nsrc, ctx->stream);
-        if (ctx->blk[from].smem)
+        if (uses_block_step(ctx))
             launch_step_block32(step32_args(ctx, from), block_step(ctx, from, blocks), ctx->dirs32t.as<DirTable>(), curved,
                                 ctx->stream);
         else if (!is_adaptive(ctx))
@@ -1435,6 +1439,7 @@ int grlbm_create(const grlbm_grid_desc *grid, const grlbm_metric_desc *metric, c
         if ((ctx->fast64 ? prepare_step64() : prepare_step32()) != cudaSuccess)
             return fail(nullptr, GRLBM_ERR_CUDA, "cannot reserve shared memory for the tiled step");
         TRY(default_step32_tile(ctx));
+        TRY(set_block_step(ctx));
     }
     if (is_adaptive(ctx))
     {
@@ -2302,7 +2307,12 @@ int grlbm_set_tile_shape(grlbm_ctx *ctx, int32_t tile_x, int32_t tile_y)
                     "tiles are a setting of the fixed streaming step of the precision and fast FP64 forms");
     cudaSetDevice(ctx->device);
     CU(cudaStreamSynchronize(ctx->stream));
-    return set_step32_tile(ctx, tile_x, tile_y);
+    if (tile_x == 0 && tile_y == 0) // the default step again
+        return default_step32_tile(ctx);
+    const int rc = set_step32_tile(ctx, tile_x, tile_y);
+    if (rc == GRLBM_OK)
+        ctx->tile_asked = true;
+    return rc;
 }
 
 int grlbm_get_tile_shape(const grlbm_ctx *ctx, int32_t *tile_x, int32_t *tile_y)
@@ -2311,8 +2321,9 @@ int grlbm_get_tile_shape(const grlbm_ctx *ctx, int32_t *tile_x, int32_t *tile_y)
         return GRLBM_ERR_ARGUMENT;
     if (!is_tiled(ctx))
         return GRLBM_ERR_UNSUPPORTED;
-    *tile_x = ctx->tile_x;
-    *tile_y = ctx->tile_y;
+    const bool own = ctx->tile_asked || ctx->tile_tuned; // (else the default step's)
+    *tile_x = own ? ctx->tile_x : 0;
+    *tile_y = own ? ctx->tile_y : 0;
     return GRLBM_OK;
 }
 
@@ -2619,7 +2630,7 @@ int batch_build(grlbm_batch *b)
     for (int k = 0; k < n; k++)
     {
         const grlbm_ctx *c = b->ctx[order[k]];
-        const int own = c->blk[0].smem ? c->blk[0].resident : c->step_blocks;
+        const int own = uses_block_step(c) ? c->blk[0].resident : c->step_blocks;
         if (b->blocks_per_sm < 0 && is_tiled(c)) // the other forms' grids cover their work once
             b->grid[k] = std::max(1, std::min(own, (int)std::ceil(-b->blocks_per_sm * own * batch_cost(c) / wsum)));
     }
@@ -2947,8 +2958,12 @@ int grlbm_batch_autotune(grlbm_batch *b, int32_t trial_steps, int32_t *blocks_pe
         for (auto &cls : classes)
         {
             grlbm_ctx *c0 = cls.second[0];
+            // the fastest so far: the tile, and whether a context's own step
+            // runs on it.  The persistent launch always does; the contexts'
+            // own steps, which it leaves alone, then stay as they were.
+            const bool own_steps = b->blocks_per_sm <= 0;
             int bx = c0->tile_x, by = c0->tile_y;
-            bool block = c0->blk[0].smem != 0; // the fastest so far is the block step
+            bool asked = c0->tile_asked, tuned = c0->tile_tuned;
             double wc = 0.0;
             for (grlbm_ctx *c : cls.second)
                 wc += batch_cost(c);
@@ -2956,7 +2971,7 @@ int grlbm_batch_autotune(grlbm_batch *b, int32_t trial_steps, int32_t *blocks_pe
                 continue;
             for (const auto &t : cand)
             {
-                if (!block && t[0] == bx && t[1] == by)
+                if ((asked || !own_steps) && t[0] == bx && t[1] == by)
                     continue;
                 size_t smem = 0;
                 int per_sm = 0;
@@ -2965,21 +2980,29 @@ int grlbm_batch_autotune(grlbm_batch *b, int32_t trial_steps, int32_t *blocks_pe
                 if (smem > (size_t)kStep32MaxSmem || per_sm < 1)
                     continue;
                 for (grlbm_ctx *c : cls.second)
+                {
                     if ((rc = set_step32_tile(c, t[0], t[1])))
                         break;
+                    c->tile_asked |= own_steps;
+                }
                 if (rc)
                     break;
                 const float ms = batch_time(b, trial_steps, e0, e1, &rc);
                 if (rc)
                     break;
                 if (ms < best)
-                    best = ms, bx = t[0], by = t[1], block = false;
+                    best = ms, bx = t[0], by = t[1], asked = tuned = true;
             }
             if (rc)
                 break;
             for (grlbm_ctx *c : cls.second)
-                if ((rc = set_step32_tile(c, bx, by)) || (block && (rc = set_block_step(c))))
+            {
+                if ((rc = set_step32_tile(c, bx, by)))
                     break;
+                if (own_steps)
+                    c->tile_asked = asked;
+                c->tile_tuned = tuned;
+            }
             if (rc)
                 break;
         }

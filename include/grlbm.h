@@ -291,16 +291,23 @@ int grlbm_node_row_bytes(const grlbm_ctx *ctx, int32_t what, int64_t *bytes);
 int grlbm_copy_node_rows(grlbm_ctx *ctx, int32_t what, int64_t j_first, int64_t n, void *buffer, int32_t to_buffer);
 /* ---- tiles of the tiled steps -----------------------------------------------
  * No counterpart in the reference.  The GRLBM_PRECISION_FP32 and
- * GRLBM_FAST_FP64 steps of the fixed streaming types run as warps that each
- * take tiles of tile_x x tile_y cells (at most 16), staging each tile's
- * (tile_x + 2) x (tile_y + 2) node patch of the state in shared memory.  The
- * default tile maximises its cells times the kernel's resident blocks per SM
- * (counted up to three), over 8x2, 4x4, 16x1, 4x3, 3x4, 4x2, 2x4, 3x3, 2x2,
- * 2x1, 1x1 in that order of preference; on small grids, with fewer 16-cell
- * tiles than 0.4 (0.2) times the warps then resident, over the tiles of at
- * most 12 (8) cells.  The result does not depend on the tile.
- * GRLBM_ERR_ARGUMENT for more than 16 cells or buffers that do not fit in
- * shared memory; GRLBM_ERR_UNSUPPORTED for other contexts. */
+ * GRLBM_FAST_FP64 steps of the fixed streaming types have two kernels: blocks
+ * of 8 warps that share the staged node patch of 8 x 8 (or 4 x 8) cells, and
+ * warps that each take tiles of tile_x x tile_y cells (at most 16), staging
+ * each tile's (tile_x + 2) x (tile_y + 2) node patch of the state in shared
+ * memory.  By default (tile 0 x 0) a step runs the first, and the second where
+ * the first's patch does not fit; setting a tile makes it run the second on
+ * that tile, setting 0 x 0 restores the default.  The result does not depend
+ * on either.  grlbm_get_tile_shape reports the tile in force, 0 x 0 for the
+ * default.  The default step's own tile, for where it runs the second kernel
+ * and for the persistent batch launch, maximises its cells times the kernel's
+ * resident blocks per SM (counted up to three), over 8x2, 4x4, 16x1, 4x3, 3x4,
+ * 4x2, 2x4, 3x3, 2x2, 2x1, 1x1 in that order of preference; on small grids,
+ * with fewer 16-cell tiles than 0.4 (0.2) times the warps then resident, over
+ * the tiles of at most 12 (8) cells.
+ * GRLBM_ERR_ARGUMENT for other tiles of less than one or more than 16 cells
+ * and for buffers that do not fit in shared memory; GRLBM_ERR_UNSUPPORTED for
+ * other contexts. */
 int grlbm_set_tile_shape(grlbm_ctx *ctx, int32_t tile_x, int32_t tile_y);
 int grlbm_get_tile_shape(const grlbm_ctx *ctx, int32_t *tile_x, int32_t *tile_y);
 /* The most node rows away from its cell that any stream gather reads: the
@@ -355,7 +362,9 @@ int grlbm_batch_set_shape(grlbm_batch *batch, int32_t blocks_per_sm, int32_t lar
  * one form, grid size and direction count) holding at least 2% of the
  * batch's estimated cost, largest class first, times candidate tile shapes
  * (grlbm_set_tile_shape) with the other classes fixed and keeps the
- * fastest.  Every problem is put back in the state it had before the
+ * fastest, the tile or default step in force before the call among them (in
+ * the persistent launch, whose tiles leave the problems' own steps as they
+ * were, the tile).  Every problem is put back in the state it had before the
  * call.  The launch shape is returned in *blocks_per_sm and *largest_first
  * (either may be NULL), the tiles by grlbm_get_tile_shape. */
 int grlbm_batch_autotune(grlbm_batch *batch, int32_t trial_steps, int32_t *blocks_per_sm, int32_t *largest_first);
