@@ -90,7 +90,11 @@ struct grlbm_ctx
     // persistent grid, and the TMA maps of the state buffers for that tile
     int tile_x = 4, tile_y = 4, passes = 1, step_blocks = 1;
     CUtensorMap in_map[2];
-    BlockStep blk[2] = {}; // blk[k]: the one-patch-per-block step that reads buffer k (smem 0: it does not fit)
+    // blk[k][r]: the one-patch-per-block step that reads buffer k, in runs of 8
+    // (r = 0) or 4 cells (smem 0: it does not fit); runs of 8 from this many of
+    // their tiles on, and the warp-per-tile kernel from this many cells on
+    BlockStep blk[2][2] = {};
+    int64_t blk_long_tiles = 0, blk_cells = 0;
     bool tile_asked = false; // a tile was asked for: the step runs the warp-per-tile kernel
     bool tile_tuned = false; // the tile is not the default one
     cudaEvent_t landed[2] = {nullptr, nullptr}; // a half of a read-back buffer has landed
@@ -608,62 +612,103 @@ int adaptive_departure_rows(grlbm_ctx *ctx, int32_t *rows)
     return GRLBM_OK;
 }
 
+// Interior cells from which the default step is the warp-per-tile kernel,
+// whose set-up is paid once a warp and not once a tile: measured at 200^2 to
+// 1000^2 with 4 to 96 directions, block against warp per tile.
+// FP32 flat, up to 64 directions (600^2: 8 directions 65.6 against 50.0 us, 32:
+// 73.8 against 70.3, 64: 98.4 against 96.7; 72 and more: the block step), from
+// fewer cells where they are odd, since the block step then stores one
+// direction a lane (400^2 x 33: 45.2 against 42.1 us; x 48: 40.9 against 43.5).
+// FP32 curved, where the directions nearly fill its half warps or warps (400^2
+// x 12: 41.0 against 37.4 us, 600^2 x 28: 117 against 111; 600^2 x 20: the block
+// step by 7%, x 36: by 25%).
+// Fast FP64 curved, at the top of its one-pass range (400^2 x 28: 112 against
+// 109 us, x 32: 108 against 98; x 33: the block step by 17%); flat: the block
+// step by 5% to 40%.
+int64_t warp_tile_cells(int nd, bool curved, bool fast64)
+{
+    constexpr int64_t never = INT64_MAX;
+    if (fast64)
+        return curved && nd > 24 && nd <= 32 ? 100000 : never;
+    if (curved)
+    {
+        if (nd <= 16)
+            return nd <= 8 ? 200000 : 100000;
+        if (nd > 24 && nd <= 32)
+            return nd < 32 ? 120000 : 500000;
+        return nd == 63 || nd == 64 ? 250000 : never;
+    }
+    if (nd > 64)
+        return never;
+    if (nd < 6)
+        return 60000;
+    if (nd & 1)
+        return 90000;
+    return nd <= 26 ? 110000 : (nd <= 34 ? 160000 : (nd <= 40 ? 200000 : 300000));
+}
+
 // Sets up the one-patch-per-block step, the default where its patch fits an
-// SM (the warp-per-tile kernel runs while a tile shape is asked for, in the
-// persistent batch launch, and for the direction counts whose patch does not
-// fit).  A warp takes 8 cells of a row, or 4 where 8 would leave the GPU
-// idle: at most one tile for every second SM (64^2 x 64 directions, fast FP64:
-// 8.2 against 9.0 us), or one block an SM where 4 give two (100^2 x 200:
-// FP32 29.6 against 38.2 us, fast FP64 53 against 92 us; 200^2 x 96 in fast
-// FP64: 73 against 80 us).  Elsewhere 8: a run's fixed work is halved (400^2 x
-// 64: FP32 82 against 105 us, fast FP64 154 against 191 us).
+// SM, up to warp_tile_cells (the warp-per-tile kernel runs from there on, while
+// a tile shape is asked for, in the persistent batch launch, and for the
+// direction counts whose patch does not fit).  A warp takes 8 cells of a row,
+// or 4 where 8 would leave the GPU idle: at most one tile for every second SM
+// (64^2 x 64 directions, fast FP64: 8.2 against 9.0 us), or one block an SM
+// where 4 give two (100^2 x 200: FP32 29.6 against 38.2 us, fast FP64 53 against
+// 92 us; 200^2 x 96 in fast FP64: 73 against 80 us).  Elsewhere 8: a run's fixed
+// work is halved (400^2 x 64: FP32 82 against 105 us, fast FP64 154 against 191
+// us).  Both lines are taken for the rows of each launch, so that a band and
+// its edge rows run as a grid of their size would.
 int set_block_step(grlbm_ctx *ctx)
 {
     const bool curved = ctx->run.streaming_type == GRLBM_CURVED_FIXED;
     const int dp = (int)ctx->sl.sp;
-    int sms = 0;
+    int sms = 0, per_sm[2] = {0, 0};
     CU(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device));
-    BlockStep b[2] = {}; // runs of 8, of 4
-    int per_sm[2] = {0, 0};
-    for (int k = 0; k < 2; k++)
+    for (int r = 0; r < 2; r++)
     {
-        b[k].run = k ? 4 : 8;
+        BlockStep b{};
+        b.run = r ? 4 : 8;
         if (ctx->fast64)
-            block_layout64(b[k], ctx->st.n, dp, ctx->dirs.q, curved);
+            block_layout64(b, ctx->st.n, dp, ctx->dirs.q, curved);
         else
-            block_layout32(b[k], ctx->st.n, dp, ctx->dirs.q, curved);
-        if (b[k].smem <= kStep32MaxSmem)
-            CU(ctx->fast64 ? block_occupancy64(curved, b[k].run, b[k].smem, &per_sm[k])
-                           : block_occupancy32(curved, b[k].run, b[k].smem, &per_sm[k]));
+            block_layout32(b, ctx->st.n, dp, ctx->dirs.q, curved);
+        if (b.smem > kStep32MaxSmem)
+            continue;
+        CU(ctx->fast64 ? block_occupancy64(curved, b.run, b.smem, &per_sm[r])
+                       : block_occupancy32(curved, b.run, b.smem, &per_sm[r]));
+        b.resident = per_sm[r] * sms;
+        for (int k = 0; k < 2 && per_sm[r] > 0; k++)
+        {
+            const cudaError_t e = ctx->fast64 ? encode_state_map64(&b.map, ctx->I[k].as<double>(), ctx->geo.nx,
+                                                                   ctx->geo.ny, dp, b.run, kBlockStepWarps)
+                                              : encode_state_map32(&b.map, ctx->I[k].as<float>(), ctx->geo.nx,
+                                                                   ctx->geo.ny, dp, b.run, kBlockStepWarps);
+            if (e != cudaSuccess)
+                return fail(ctx, GRLBM_ERR_CUDA, "TMA map of the state: %s", cudaGetErrorString(e));
+            ctx->blk[k][r] = b;
+        }
     }
-    const int64_t tiles = ((ctx->gd.nx_ + 7) / 8) * ((ctx->gd.jhi - ctx->gd.jlo + kBlockStepWarps - 1) / kBlockStepWarps);
-    const int pick = per_sm[0] < 1 || (per_sm[0] == 1 && per_sm[1] > 1) || 2 * tiles <= sms ? 1 : 0;
-    if (per_sm[pick] < 1)
-        return GRLBM_OK;
-    for (int k = 0; k < 2; k++)
-    {
-        ctx->blk[k] = b[pick];
-        ctx->blk[k].resident = per_sm[pick] * sms;
-        const cudaError_t e = ctx->fast64 ? encode_state_map64(&ctx->blk[k].map, ctx->I[k].as<double>(), ctx->geo.nx,
-                                                               ctx->geo.ny, dp, b[pick].run, kBlockStepWarps)
-                                          : encode_state_map32(&ctx->blk[k].map, ctx->I[k].as<float>(), ctx->geo.nx,
-                                                               ctx->geo.ny, dp, b[pick].run, kBlockStepWarps);
-        if (e != cudaSuccess)
-            return fail(ctx, GRLBM_ERR_CUDA, "TMA map of the state: %s", cudaGetErrorString(e));
-    }
+    ctx->blk_long_tiles = per_sm[0] < 1 || (per_sm[0] == 1 && per_sm[1] > 1) ? INT64_MAX : sms / 2 + 1;
+    ctx->blk_cells = warp_tile_cells(ctx->st.n, curved, ctx->fast64);
     return GRLBM_OK;
 }
 
-// The block step's tiles over the rows of the context's band, on a grid of
-// `blocks` (0: one a tile).
-bool uses_block_step(const grlbm_ctx *ctx) { return ctx->blk[0].smem && !ctx->tile_asked; }
+// The block step over the rows of the context's band, on a grid of `blocks`
+// (0: one a tile); smem 0: the step runs the warp-per-tile kernel.
 BlockStep block_step(const grlbm_ctx *ctx, int from, int blocks)
 {
-    BlockStep b = ctx->blk[from];
-    b.grid = blocks;
     const int64_t rows = ctx->gd.jhi - ctx->gd.jlo;
+    auto tiles = [rows](int64_t w, int run) {
+        return rows <= 0 ? 0 : (w + run - 1) / run * ((rows + kBlockStepWarps - 1) / kBlockStepWarps);
+    };
+    if (ctx->tile_asked || ctx->gd.nx_ * rows >= ctx->blk_cells)
+        return BlockStep{};
+    BlockStep b = ctx->blk[from][tiles(ctx->gd.nx_, 8) < ctx->blk_long_tiles];
+    if (!b.smem)
+        return b;
+    b.grid = blocks;
     b.tiles_x = (int)((ctx->gd.nx_ + b.run - 1) / b.run);
-    b.tiles_y = rows <= 0 ? 0 : (int)((rows + kBlockStepWarps - 1) / kBlockStepWarps);
+    b.tiles_y = (int)(tiles(1, b.run));
     return b;
 }
 
@@ -800,9 +845,8 @@ int enqueue_step(grlbm_ctx *ctx, int from, bool sources = true, int blocks = 0)
         if (sources && ctx->run.keep_source_nodes_active && ctx->nsrc > 0)
             launch_sources64L(ctx->I[from].as<double>(), ctx->sl, ctx->st.n, ctx->src_nodes.as<int64_t>(),
                               ctx->src_vals.as<double>(), ctx->nsrc, ctx->stream);
-        if (uses_block_step(ctx))
-            launch_step_block64(step64_args(ctx, from), block_step(ctx, from, blocks), ctx->dirs64t.as<DirTable64>(), curved,
-                                ctx->stream);
+        if (const BlockStep b = block_step(ctx, from, blocks); b.smem)
+            launch_step_block64(step64_args(ctx, from), b, ctx->dirs64t.as<DirTable64>(), curved, ctx->stream);
         else
             launch_step64(step64_args(ctx, from), ctx->dirs64t.as<DirTable64>(), curved, ctx->passes,
                           tile_blocks, ctx->stream);
@@ -812,9 +856,8 @@ int enqueue_step(grlbm_ctx *ctx, int from, bool sources = true, int blocks = 0)
         if (sources && ctx->run.keep_source_nodes_active && ctx->nsrc > 0)
             launch_sources32(ctx->I[from].as<float>(), ctx->sl, ctx->st.n, ctx->src_nodes.as<int64_t>(),
                              ctx->src_vals.as<float>(), ctx->nsrc, ctx->stream);
-        if (uses_block_step(ctx))
-            launch_step_block32(step32_args(ctx, from), block_step(ctx, from, blocks), ctx->dirs32t.as<DirTable>(), curved,
-                                ctx->stream);
+        if (const BlockStep b = is_adaptive(ctx) ? BlockStep{} : block_step(ctx, from, blocks); b.smem)
+            launch_step_block32(step32_args(ctx, from), b, ctx->dirs32t.as<DirTable>(), curved, ctx->stream);
         else if (!is_adaptive(ctx))
             launch_step32(step32_args(ctx, from), ctx->dirs, curved, ctx->passes, tile_blocks, ctx->stream);
         else
@@ -2630,9 +2673,11 @@ int batch_build(grlbm_batch *b)
     for (int k = 0; k < n; k++)
     {
         const grlbm_ctx *c = b->ctx[order[k]];
-        const int own = uses_block_step(c) ? c->blk[0].resident : c->step_blocks;
-        if (b->blocks_per_sm < 0 && is_tiled(c)) // the other forms' grids cover their work once
-            b->grid[k] = std::max(1, std::min(own, (int)std::ceil(-b->blocks_per_sm * own * batch_cost(c) / wsum)));
+        if (b->blocks_per_sm >= 0 || !is_tiled(c)) // the other forms' grids cover their work once
+            continue;
+        const BlockStep blk = block_step(c, 0, 0);
+        const int own = blk.smem ? blk.resident : c->step_blocks;
+        b->grid[k] = std::max(1, std::min(own, (int)std::ceil(-b->blocks_per_sm * own * batch_cost(c) / wsum)));
     }
     if (alloc(nullptr, b->d_items, n * sizeof(Batch32Item)) || alloc(nullptr, b->d_first, (n + 1) * sizeof(int)))
         return bfail(b, GRLBM_ERR_CUDA, "cannot allocate the batch launch list");

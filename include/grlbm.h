@@ -296,7 +296,8 @@ int grlbm_copy_node_rows(grlbm_ctx *ctx, int32_t what, int64_t j_first, int64_t 
  * warps that each take tiles of tile_x x tile_y cells (at most 16), staging
  * each tile's (tile_x + 2) x (tile_y + 2) node patch of the state in shared
  * memory.  By default (tile 0 x 0) a step runs the first, and the second where
- * the first's patch does not fit; setting a tile makes it run the second on
+ * the first's patch does not fit or the rows stepped hold so many cells of so
+ * few directions that the second is faster; setting a tile makes it run the second on
  * that tile, setting 0 x 0 restores the default.  The result does not depend
  * on either.  grlbm_get_tile_shape reports the tile in force, 0 x 0 for the
  * default.  The default step's own tile, for where it runs the second kernel
