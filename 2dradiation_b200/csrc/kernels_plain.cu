@@ -603,7 +603,9 @@ __device__ __forceinline__ bool still_changing(const double (&p)[6], const doubl
 // sums, doubled the warps but took a third more operations: 183 us against
 // 134 at 400^2 x 64.)
 constexpr int kColumnTileY = 4; // 16 x 4 cells per block with COLUMN
-constexpr int kColumnMaxDirs = 90; // the column and the tables within 48 KB
+// the column up to 91 directions (100^2 x 91 flat: 39 us a step against 69
+// without it)
+constexpr int kColumnMaxDirs = 91;
 #ifndef GRLBM_COLLIDE_MIN_BLOCKS
 #define GRLBM_COLLIDE_MIN_BLOCKS 6
 #endif
@@ -1116,6 +1118,10 @@ cudaError_t prepare_step_plain(int smem_bytes)
     limit((const void *)k_stream_plain_patch<true, 4>, patch);
     limit((const void *)k_stream_plain_patch<false, 6>, patch);
     limit((const void *)k_stream_plain_patch<true, 6>, patch);
+    const int column = (int)collide_smem(kColumnMaxDirs, true);
+    limit((const void *)k_collide_plain<false, false, true>, column);
+    limit((const void *)k_collide_plain<false, true, true>, column);
+    limit((const void *)k_collide_plain<true, false, true>, column);
     return e;
 }
 void launch_step_plain(const PlainStepArgs &a, bool curved, cudaStream_t s, const StepRecord *record)
@@ -1166,7 +1172,6 @@ void launch_step_plain(const PlainStepArgs &a, bool curved, cudaStream_t s, cons
     const dim3 kgrid(tx, column ? nblk(a.g.jhi - a.g.jlo, kColumnTileY) : ty);
     const unsigned kthreads = column ? kSplitTileX * kColumnTileY : kStepBlock;
     const size_t ksmem = collide_smem(a.nd, column);
-    static_assert(collide_smem(kColumnMaxDirs, true) <= 48 * 1024, "within the default limit");
     if (adaptive)
         column ? k_collide_plain<false, true, true><<<kgrid, kthreads, ksmem, s>>>(a, rec)
                : k_collide_plain<false, true, false><<<kgrid, kthreads, ksmem, s>>>(a, rec);
