@@ -235,6 +235,14 @@ struct __align__(16) IgRow32
     float4 w;
 };
 
+// What the nodes' fluid asks of the plain collide: nothing moves or scatters
+// anisotropically, some node scatters anisotropically, some node moves.
+enum Fluid
+{
+    FLUID_AT_REST,
+    FLUID_ANISOTROPIC,
+    FLUID_MOVING
+};
 struct PlainStepArgs
 {
     GridDev g;
@@ -249,6 +257,7 @@ struct PlainStepArgs
     const double *acube;       // nxy*9
     const uint8_t *flags;      // nxy: bit0 excised node (no collide), bit1 stream writes 0
     const double *u1, *u2, *lor, *adt, *eta, *k0, *k3, *ka; // k3 = 3 kappa1
+    int fluid;                 // Fluid: the most general node's
     double *mom;               // 6*nxy
     unsigned long long *iter_sum;
     unsigned int *iter_max;

@@ -95,6 +95,7 @@ struct grlbm_ctx
     // their tiles on, and the warp-per-tile kernel from this many cells on
     BlockStep blk[2][2] = {};
     int64_t blk_long_tiles = 0, blk_cells = 0;
+    Fluid fluid = FLUID_AT_REST; // the most general node's
     bool tile_asked = false; // a tile was asked for: the step runs the warp-per-tile kernel
     bool tile_tuned = false; // the tile is not the default one
     cudaEvent_t landed[2] = {nullptr, nullptr}; // a half of a read-back buffer has landed
@@ -798,6 +799,7 @@ PlainStepArgs plain_args(grlbm_ctx *ctx, int from)
     a.adt = ctx->cadt.as<double>();
     a.eta = ctx->ceta.as<double>();
     a.k0 = ctx->ck0.as<double>();
+    a.fluid = ctx->fluid;
     a.k3 = ctx->ck3.as<double>();
     a.ka = ctx->cka.as<double>();
     a.mom = ctx->mom.as<double>();
@@ -1557,6 +1559,7 @@ int grlbm_set_fields(grlbm_ctx *ctx, const double *kappa0, const double *kappa1,
     const int64_t nxy = ctx->geo.nxy;
     const MetricArrays &M = ctx->M;
     std::vector<double> u1(nxy), u2(nxy), lor(nxy), adt(nxy), k3(nxy);
+    Fluid fluid = FLUID_AT_REST;
     for (int64_t ij = 0; ij < nxy; ij++)
     {
         // TransformLFtoIF(uLF, GetTetrad(ij)) as Collide calls it (src/Radiation.cpp:652-657)
@@ -1567,7 +1570,12 @@ int grlbm_set_fields(grlbm_ctx *ctx, const double *kappa0, const double *kappa1,
         lor[ij] = 1.0 / std::sqrt(1.0 - (a * a + b * b));
         adt[ij] = M.at(ALPHA, ij) * ctx->geo.dt;
         k3[ij] = 3.0 * kappa1[ij];
+        if (!(a == 0.0 && b == 0.0))
+            fluid = FLUID_MOVING;
+        else if (k3[ij] != 0.0)
+            fluid = std::max(fluid, FLUID_ANISOTROPIC);
     }
+    ctx->fluid = fluid;
     int rc;
     if ((rc = upload_t(ctx, ctx->cu1, u1)) || (rc = upload_t(ctx, ctx->cu2, u2)) ||
         (rc = upload_t(ctx, ctx->clor, lor)) || (rc = upload_t(ctx, ctx->cadt, adt)) ||

@@ -604,10 +604,21 @@ __device__ __forceinline__ bool still_changing(const double (&p)[6], const doubl
 // 134 at 400^2 x 64.)
 constexpr int kColumnTileY = 4; // 16 x 4 cells per block with COLUMN
 // the column up to 91 directions (100^2 x 91 flat: 39 us a step against 69
-// without it)
-constexpr int kColumnMaxDirs = 91;
+// without it), 90 for a moving fluid (400 x 300 x 91: 1125 against 727)
+constexpr int kColumnMaxDirs = 91, kColumnMaxDirsMoving = 90;
+// Resident blocks the kernel with the column is compiled for.  A fluid at rest
+// without anisotropic scattering: 6 (142 registers; 8 blocks are 2% to 5%
+// slower).  GENERAL, a fluid that moves or scatters anisotropically somewhere,
+// whose passes are chains of divisions: 8 (128 registers; 400 x 300 x 48 moving,
+// flat: 381 us a step against 474 with 6, x 33 anisotropic: 90 against 103).
 #ifndef GRLBM_COLLIDE_MIN_BLOCKS
 #define GRLBM_COLLIDE_MIN_BLOCKS 6
+#endif
+#ifndef GRLBM_COLLIDE_GENERAL_BLOCKS
+#define GRLBM_COLLIDE_GENERAL_BLOCKS 8
+#endif
+#ifndef GRLBM_COLLIDE_WIDE_BLOCKS
+#define GRLBM_COLLIDE_WIDE_BLOCKS 4
 #endif
 #ifndef GRLBM_COLLIDE_UNROLL
 #define GRLBM_COLLIDE_UNROLL 8
@@ -617,8 +628,10 @@ constexpr size_t collide_smem(int nd, bool column)
 {
     return (size_t)nd * (4 + (column ? kSplitTileX * kColumnTileY : 0)) * sizeof(double);
 }
-template <bool RECORD, bool ADAPTIVE, bool COLUMN>
-__global__ void __launch_bounds__(COLUMN ? kSplitTileX *kColumnTileY : kStepBlock, COLUMN ? GRLBM_COLLIDE_MIN_BLOCKS : 4)
+template <bool RECORD, bool ADAPTIVE, bool COLUMN, bool GENERAL = false>
+__global__ void __launch_bounds__(COLUMN ? kSplitTileX *kColumnTileY : kStepBlock,
+                                  !COLUMN ? GRLBM_COLLIDE_WIDE_BLOCKS
+                                          : (GENERAL ? GRLBM_COLLIDE_GENERAL_BLOCKS : GRLBM_COLLIDE_MIN_BLOCKS))
     k_collide_plain(const __grid_constant__ PlainStepArgs a, const __grid_constant__ StepRecord rec)
 {
     constexpr int TY = COLUMN ? kColumnTileY : kSplitTileY, NT = kSplitTileX * TY;
@@ -761,11 +774,14 @@ __global__ void __launch_bounds__(COLUMN ? kSplitTileX *kColumnTileY : kStepBloc
                 }
             }
             else if (rest)
+            {
+#pragma unroll 4
                 for (int d = 0; d < nd; d++)
                 {
                     const double2 n = direction(d);
                     m.add(dir[2 * d + 1].x, value(d, n), n.x, n.y);
                 }
+            }
             else
                 for (int d = 0; d < nd; d++)
                 {
@@ -786,8 +802,11 @@ __global__ void __launch_bounds__(COLUMN ? kSplitTileX *kColumnTileY : kStepBloc
                 out[(int64_t)d * nxy] = quotient_plain(streamed(d) + src);
         }
         else if (rest)
+        {
+#pragma unroll 4
             for (int d = 0; d < nd; d++)
                 out[(int64_t)d * nxy] = value(d, direction(d));
+        }
         else
             for (int d = 0; d < nd; d++)
             {
@@ -1120,7 +1139,9 @@ cudaError_t prepare_step_plain(int smem_bytes)
     limit((const void *)k_stream_plain_patch<true, 6>, patch);
     const int column = (int)collide_smem(kColumnMaxDirs, true);
     limit((const void *)k_collide_plain<false, false, true>, column);
+    limit((const void *)k_collide_plain<false, false, true, true>, column);
     limit((const void *)k_collide_plain<false, true, true>, column);
+    limit((const void *)k_collide_plain<false, true, true, true>, column);
     limit((const void *)k_collide_plain<true, false, true>, column);
     return e;
 }
@@ -1168,19 +1189,22 @@ void launch_step_plain(const PlainStepArgs &a, bool curved, cudaStream_t s, cons
         record ? k_stream_plain<false, true, false><<<gf, kStepBlock, 0, s>>>(a, rec)
                : k_stream_plain<false, false, false><<<gf, kStepBlock, 0, s>>>(a, rec);
     // moments and collide: with each cell's values in shared memory when they fit
-    const bool column = a.nd <= kColumnMaxDirs;
+    const bool column = a.nd <= (a.fluid == FLUID_MOVING ? kColumnMaxDirsMoving : kColumnMaxDirs);
     const dim3 kgrid(tx, column ? nblk(a.g.jhi - a.g.jlo, kColumnTileY) : ty);
     const unsigned kthreads = column ? kSplitTileX * kColumnTileY : kStepBlock;
     const size_t ksmem = collide_smem(a.nd, column);
-    if (adaptive)
-        column ? k_collide_plain<false, true, true><<<kgrid, kthreads, ksmem, s>>>(a, rec)
-               : k_collide_plain<false, true, false><<<kgrid, kthreads, ksmem, s>>>(a, rec);
-    else if (record)
+    if (record && !adaptive)
         column ? k_collide_plain<true, false, true><<<kgrid, kthreads, ksmem, s>>>(a, rec)
                : k_collide_plain<true, false, false><<<kgrid, kthreads, ksmem, s>>>(a, rec);
+    else if (!column)
+        adaptive ? k_collide_plain<false, true, false><<<kgrid, kthreads, ksmem, s>>>(a, rec)
+                 : k_collide_plain<false, false, false><<<kgrid, kthreads, ksmem, s>>>(a, rec);
+    else if (adaptive)
+        a.fluid != FLUID_AT_REST ? k_collide_plain<false, true, true, true><<<kgrid, kthreads, ksmem, s>>>(a, rec)
+                  : k_collide_plain<false, true, true><<<kgrid, kthreads, ksmem, s>>>(a, rec);
     else
-        column ? k_collide_plain<false, false, true><<<kgrid, kthreads, ksmem, s>>>(a, rec)
-               : k_collide_plain<false, false, false><<<kgrid, kthreads, ksmem, s>>>(a, rec);
+        a.fluid != FLUID_AT_REST ? k_collide_plain<false, false, true, true><<<kgrid, kthreads, ksmem, s>>>(a, rec)
+                  : k_collide_plain<false, false, true><<<kgrid, kthreads, ksmem, s>>>(a, rec);
     if (adaptive) // the halo moments, recomputed by the reference from unwritten (zero) intensities
         k_zero_halo_moments<double><<<nblk(a.g.nxy, 256), 256, 0, s>>>(a.g, a.mom);
 }
