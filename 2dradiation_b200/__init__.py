@@ -490,17 +490,17 @@ def batch_cost(case: dict, precision: int = PRECISION_FP32) -> float:
     """A problem's estimated step time in arbitrary units, as a batch's
     launch shares estimate it (grlbm_batch_set_shape): cells x (directions +
     48), x 1.6 for curved streaming, x the form's cost against the FP32
-    fixed-streaming step (fast FP64 1.9, plain FP64 4.7, adaptive streaming
-    4.9 in FP32 and 10.9 in plain FP64)."""
+    fixed-streaming step (fast FP64 1.9, plain FP64 2.6, adaptive streaming
+    4.6 in FP32 and 12.2 in plain FP64)."""
     st = int(case["streaming_type"])
     curved = st in (CURVED_FIXED, CURVED_ADAPTIVE)
     adaptive = st in (FLAT_ADAPTIVE, CURVED_ADAPTIVE)
     if precision == FAST_FP64:
         form = 1.9
     elif adaptive:
-        form = 4.9 if precision == PRECISION_FP32 else 10.9
+        form = 4.6 if precision == PRECISION_FP32 else 12.2
     else:
-        form = 1.0 if precision == PRECISION_FP32 else 4.7
+        form = 1.0 if precision == PRECISION_FP32 else 2.6
     return int(case["nx_"]) * int(case["ny_"]) * (int(case["n_dir"]) + 48.0) * (1.6 if curved else 1.0) * form
 
 

@@ -2584,11 +2584,12 @@ void batch_drop_graphs(grlbm_batch *b)
 
 // A problem's estimated step time in arbitrary units: its cells times (its
 // directions + 48), times 1.6 for curved streaming, times its form's cost
-// against the FP32 fixed-streaming step.  The FP32 step's rates at 512^2 with
-// 16, 32 and 64 directions fit a per-cell cost of a + b nd with a between 40
-// and 57 b, curved streaming 1.5-1.75 times flat; at 400^2 x 64 the fast FP64
-// step takes 1.9 times as long, the plain FP64 step 4.7 times, and adaptive
-// streaming 4.9 (FP32) and 10.9 (plain) times.
+// against the FP32 fixed-streaming step.  The FP32 step's times at 256^2 and
+// 400^2 with 16, 32 and 64 directions fit a per-cell cost of a + b nd with a
+// between 26 and 61 b, curved streaming 1.2-1.8 times flat; at 400^2 x 64,
+// curved, the fast FP64 step takes 1.9 times as long (156 against 84 us), the
+// plain FP64 step 2.6 times (222 us), and adaptive streaming 4.6 (FP32, 390 us)
+// and 12.2 (plain, 1027 us) times.
 double batch_cost(const grlbm_ctx *c)
 {
     const bool curved = is_curved(c);
@@ -2596,9 +2597,9 @@ double batch_cost(const grlbm_ctx *c)
     if (c->fast64)
         form = 1.9;
     else if (is_adaptive(c))
-        form = c->fp32 ? 4.9 : 10.9;
+        form = c->fp32 ? 4.6 : 12.2;
     else if (!c->fp32)
-        form = 4.7;
+        form = 2.6;
     return (double)c->ncell * (c->st.n + 48.0) * (curved ? 1.6 : 1.0) * form;
 }
 
