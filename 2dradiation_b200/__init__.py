@@ -88,6 +88,7 @@ SIGNATURES = {
     "grlbm_energy_noalloc": ([C.c_void_p, C.c_int64, C.c_int64, C.c_void_p, C.c_void_p], C.c_int),
     "grlbm_selftest_staging_wait": ([C.c_int32, C.c_int32, C.c_int32, C.POINTER(C.c_int32),
                                      C.POINTER(C.c_double)], C.c_int),
+    "grlbm_selftest_step_kernel": ([C.c_void_p] + [C.POINTER(C.c_int32)] * 3, C.c_int),
     "grlbm_get_stats": ([C.c_void_p, C.POINTER(Stats)], C.c_int),
     "grlbm_batch_create": ([C.POINTER(C.c_void_p), C.c_int32, C.POINTER(C.c_void_p)], C.c_int),
     "grlbm_batch_destroy": ([C.c_void_p], None),
@@ -364,6 +365,13 @@ class Radiation:
         x, y = C.c_int32(), C.c_int32()
         self._c(lib().grlbm_get_tile_shape(self.h, C.byref(x), C.byref(y)))
         return (x.value, y.value)
+
+    def step_kernel(self) -> dict:
+        """Which kernel the step last enqueued runs (grlbm_selftest_step_kernel)."""
+        k, d, b = C.c_int32(), C.c_int32(), C.c_int32()
+        self._c(lib().grlbm_selftest_step_kernel(self.h, C.byref(k), C.byref(d), C.byref(b)))
+        name = {0: None, 1: "block", 2: "warp", 3: "plain", 4: "adaptive_fp32"}[k.value]
+        return {"kernel": name, "detail": d.value, "blocks": b.value}
 
     def departure_rows(self) -> int:
         v = C.c_int32()

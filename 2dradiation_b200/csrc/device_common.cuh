@@ -475,14 +475,18 @@ void launch_departure(const DepartureArgs &a, cudaStream_t s);
 void launch_alpha_cube(const GridDev &g, const double *alpha, double *acube, cudaStream_t s);
 
 cudaError_t prepare_step_plain(int smem_bytes);
-void launch_step_plain(const PlainStepArgs &a, bool curved, cudaStream_t s, const StepRecord *record = nullptr);
+// returns which collide ran: with the column (bit 0), at a general fluid's
+// resident blocks (bit 1)
+constexpr int kCollideColumn = 1, kCollideGeneral = 2;
+int launch_step_plain(const PlainStepArgs &a, bool curved, cudaStream_t s, const StepRecord *record = nullptr);
 // One block's bounded wait on an mbarrier phase nothing (arrive = 0) or one
 // arrival (arrive = 1) completes; synchronous.
 cudaError_t run_wait_selftest(int arrive, unsigned long long limit_ns, int *completed, unsigned long long *waited_ns);
 // the adaptive streaming types in the precision form: stream, then moments
-// and collide (and the rotation update before, the halo moments after)
+// and collide (and the rotation update before, the halo moments after);
+// returns whether the stream read a staged patch
 cudaError_t prepare_step_prec_adaptive();
-void launch_step_prec_adaptive(const PrecStepArgs &a, const DirTable &dt, bool curved, cudaStream_t s);
+bool launch_step_prec_adaptive(const PrecStepArgs &a, const DirTable &dt, bool curved, cudaStream_t s);
 
 // The fixed streaming types in the precision form (kernels_step32.cu).
 // Passes per lane for nd directions (an instantiated count >= nd / 32), or -1.
@@ -514,10 +518,10 @@ void launch_step_batch32(const Batch32Item *items, const int *first_tile, int n_
                          unsigned *counters, int P, int blocks, size_t smem, int warp_stride, int s_offset,
                          int item_bytes, cudaStream_t s);
 // The one-patch-per-block step (step_block.cuh): shared memory of a tile
-// (b.run set), its resident blocks per SM, and the launch.
+// (b.run set), its resident blocks per SM, and the launch (returns its blocks).
 void block_layout32(BlockStep &b, int nd, int dp, int q, bool curved);
 cudaError_t block_occupancy32(bool curved, int run, int smem, int *blocks);
-void launch_step_block32(const Step32Args &a, const BlockStep &b, const DirTable *dt, bool curved, cudaStream_t s);
+int launch_step_block32(const Step32Args &a, const BlockStep &b, const DirTable *dt, bool curved, cudaStream_t s);
 // The TMA map the step stages a cell-major state of nx x ny nodes through,
 // for tiles of tx x ty cells.
 cudaError_t encode_state_map32(CUtensorMap *map, const float *state, int64_t nx, int64_t ny, int dp, int tx, int ty);
@@ -533,7 +537,7 @@ cudaError_t prepare_step64();
 cudaError_t step64_occupancy(int P, bool curved, size_t smem, int *blocks);
 void block_layout64(BlockStep &b, int nd, int dp, int q, bool curved);
 cudaError_t block_occupancy64(bool curved, int run, int smem, int *blocks);
-void launch_step_block64(const Step64Args &a, const BlockStep &b, const DirTable64 *dt, bool curved, cudaStream_t s);
+int launch_step_block64(const Step64Args &a, const BlockStep &b, const DirTable64 *dt, bool curved, cudaStream_t s);
 void launch_step64(const Step64Args &a, const DirTable64 *dt, bool curved, int P, int blocks, cudaStream_t s);
 cudaError_t encode_state_map64(CUtensorMap *map, const double *state, int64_t nx, int64_t ny, int dp, int tx, int ty);
 

@@ -96,6 +96,7 @@ struct grlbm_ctx
     BlockStep blk[2][2] = {};
     int64_t blk_long_tiles = 0, blk_cells = 0;
     Fluid fluid = FLUID_AT_REST; // the most general node's
+    int ran[3] = {0, 0, 0};      // the step last enqueued: kernel, detail, blocks (grlbm_selftest_step_kernel)
     bool tile_asked = false; // a tile was asked for: the step runs the warp-per-tile kernel
     bool tile_tuned = false; // the tile is not the default one
     cudaEvent_t landed[2] = {nullptr, nullptr}; // a half of a read-back buffer has landed
@@ -841,6 +842,7 @@ int enqueue_step(grlbm_ctx *ctx, int from, bool sources = true, int blocks = 0)
 {
     const bool curved = is_curved(ctx);
     const int tile_blocks = blocks > 0 ? blocks : ctx->step_blocks; // the warp-per-tile kernels'
+    auto note = [ctx](int kernel, int detail, int n) { ctx->ran[0] = kernel, ctx->ran[1] = detail, ctx->ran[2] = n; };
     unsigned long long *cnt = ctx->counters.as<unsigned long long>();
     if (ctx->fast64)
     {
@@ -848,10 +850,14 @@ int enqueue_step(grlbm_ctx *ctx, int from, bool sources = true, int blocks = 0)
             launch_sources64L(ctx->I[from].as<double>(), ctx->sl, ctx->st.n, ctx->src_nodes.as<int64_t>(),
                               ctx->src_vals.as<double>(), ctx->nsrc, ctx->stream);
         if (const BlockStep b = block_step(ctx, from, blocks); b.smem)
-            launch_step_block64(step64_args(ctx, from), b, ctx->dirs64t.as<DirTable64>(), curved, ctx->stream);
+            note(GRLBM_STEP_BLOCK, b.run,
+                 launch_step_block64(step64_args(ctx, from), b, ctx->dirs64t.as<DirTable64>(), curved, ctx->stream));
         else
-            launch_step64(step64_args(ctx, from), ctx->dirs64t.as<DirTable64>(), curved, ctx->passes,
-                          tile_blocks, ctx->stream);
+        {
+            note(GRLBM_STEP_WARP_TILE, 0, tile_blocks);
+            launch_step64(step64_args(ctx, from), ctx->dirs64t.as<DirTable64>(), curved, ctx->passes, tile_blocks,
+                          ctx->stream);
+        }
     }
     else if (ctx->fp32)
     {
@@ -859,9 +865,13 @@ int enqueue_step(grlbm_ctx *ctx, int from, bool sources = true, int blocks = 0)
             launch_sources32(ctx->I[from].as<float>(), ctx->sl, ctx->st.n, ctx->src_nodes.as<int64_t>(),
                              ctx->src_vals.as<float>(), ctx->nsrc, ctx->stream);
         if (const BlockStep b = is_adaptive(ctx) ? BlockStep{} : block_step(ctx, from, blocks); b.smem)
-            launch_step_block32(step32_args(ctx, from), b, ctx->dirs32t.as<DirTable>(), curved, ctx->stream);
+            note(GRLBM_STEP_BLOCK, b.run,
+                 launch_step_block32(step32_args(ctx, from), b, ctx->dirs32t.as<DirTable>(), curved, ctx->stream));
         else if (!is_adaptive(ctx))
+        {
+            note(GRLBM_STEP_WARP_TILE, 0, tile_blocks);
             launch_step32(step32_args(ctx, from), ctx->dirs, curved, ctx->passes, tile_blocks, ctx->stream);
+        }
         else
         {
             PrecStepArgs a = prec_args(ctx, from);
@@ -873,7 +883,7 @@ int enqueue_step(grlbm_ctx *ctx, int from, bool sources = true, int blocks = 0)
             a.ang_new = ctx->ang[from ^ 1].as<double>();
             a.rot_inv = ctx->rot.as<float2>();
             a.rot_new = ctx->rot.as<float2>() + ctx->gd.nxy;
-            launch_step_prec_adaptive(a, ctx->dirs, curved, ctx->stream);
+            note(GRLBM_STEP_ADAPTIVE_FP32, launch_step_prec_adaptive(a, ctx->dirs, curved, ctx->stream) ? 1 : 0, 0);
         }
     }
     else
@@ -895,7 +905,7 @@ int enqueue_step(grlbm_ctx *ctx, int from, bool sources = true, int blocks = 0)
             a.coef = ctx->coef_k.as<double>();
             a.nf = ctx->ss.n;
         }
-        launch_step_plain(a, curved, ctx->stream);
+        note(GRLBM_STEP_PLAIN, launch_step_plain(a, curved, ctx->stream), 0);
     }
     CU(cudaGetLastError());
     return GRLBM_OK;
@@ -2375,6 +2385,16 @@ int grlbm_get_tile_shape(const grlbm_ctx *ctx, int32_t *tile_x, int32_t *tile_y)
     const bool own = ctx->tile_asked || ctx->tile_tuned; // (else the default step's)
     *tile_x = own ? ctx->tile_x : 0;
     *tile_y = own ? ctx->tile_y : 0;
+    return GRLBM_OK;
+}
+
+int grlbm_selftest_step_kernel(const grlbm_ctx *ctx, int32_t *kernel, int32_t *detail, int32_t *blocks)
+{
+    if (!ctx || !kernel || !detail || !blocks)
+        return GRLBM_ERR_ARGUMENT;
+    *kernel = ctx->ran[0];
+    *detail = ctx->ran[1];
+    *blocks = ctx->ran[2];
     return GRLBM_OK;
 }
 

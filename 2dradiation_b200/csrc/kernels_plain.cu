@@ -1145,11 +1145,11 @@ cudaError_t prepare_step_plain(int smem_bytes)
     limit((const void *)k_collide_plain<true, false, true>, column);
     return e;
 }
-void launch_step_plain(const PlainStepArgs &a, bool curved, cudaStream_t s, const StepRecord *record)
+int launch_step_plain(const PlainStepArgs &a, bool curved, cudaStream_t s, const StepRecord *record)
 {
     const int64_t cells = (a.g.jhi - a.g.jlo) * a.g.nx_;
     if (cells <= 0)
-        return;
+        return 0;
     const bool adaptive = a.ang_new != nullptr;
     const StepRecord none{};
     const StepRecord &rec = record && !adaptive ? *record : none;
@@ -1190,6 +1190,7 @@ void launch_step_plain(const PlainStepArgs &a, bool curved, cudaStream_t s, cons
                : k_stream_plain<false, false, false><<<gf, kStepBlock, 0, s>>>(a, rec);
     // moments and collide: with each cell's values in shared memory when they fit
     const bool column = a.nd <= (a.fluid == FLUID_MOVING ? kColumnMaxDirsMoving : kColumnMaxDirs);
+    const bool general = column && !record && a.fluid != FLUID_AT_REST;
     const dim3 kgrid(tx, column ? nblk(a.g.jhi - a.g.jlo, kColumnTileY) : ty);
     const unsigned kthreads = column ? kSplitTileX * kColumnTileY : kStepBlock;
     const size_t ksmem = collide_smem(a.nd, column);
@@ -1200,13 +1201,14 @@ void launch_step_plain(const PlainStepArgs &a, bool curved, cudaStream_t s, cons
         adaptive ? k_collide_plain<false, true, false><<<kgrid, kthreads, ksmem, s>>>(a, rec)
                  : k_collide_plain<false, false, false><<<kgrid, kthreads, ksmem, s>>>(a, rec);
     else if (adaptive)
-        a.fluid != FLUID_AT_REST ? k_collide_plain<false, true, true, true><<<kgrid, kthreads, ksmem, s>>>(a, rec)
-                  : k_collide_plain<false, true, true><<<kgrid, kthreads, ksmem, s>>>(a, rec);
+        general ? k_collide_plain<false, true, true, true><<<kgrid, kthreads, ksmem, s>>>(a, rec)
+                : k_collide_plain<false, true, true><<<kgrid, kthreads, ksmem, s>>>(a, rec);
     else
-        a.fluid != FLUID_AT_REST ? k_collide_plain<false, false, true, true><<<kgrid, kthreads, ksmem, s>>>(a, rec)
-                  : k_collide_plain<false, false, true><<<kgrid, kthreads, ksmem, s>>>(a, rec);
+        general ? k_collide_plain<false, false, true, true><<<kgrid, kthreads, ksmem, s>>>(a, rec)
+                : k_collide_plain<false, false, true><<<kgrid, kthreads, ksmem, s>>>(a, rec);
     if (adaptive) // the halo moments, recomputed by the reference from unwritten (zero) intensities
         k_zero_halo_moments<double><<<nblk(a.g.nxy, 256), 256, 0, s>>>(a.g, a.mom);
+    return (column ? kCollideColumn : 0) | (general ? kCollideGeneral : 0);
 }
 void launch_sources64(double *I, int64_t nxy, int nd, const int64_t *nodes, const double *vals, int64_t nsrc,
                       cudaStream_t s)

@@ -759,11 +759,12 @@ cudaError_t prepare_step_prec_adaptive()
                                 (int)kAPatchMaxSmem);
 }
 
-void launch_step_prec_adaptive(const PrecStepArgs &a, const DirTable &dt, bool curved, cudaStream_t s)
+bool launch_step_prec_adaptive(const PrecStepArgs &a, const DirTable &dt, bool curved, cudaStream_t s)
 {
     const int64_t rows = a.g.jhi - a.g.jlo;
     if (rows <= 0 || a.g.nx_ <= 0)
-        return;
+        return false;
+    bool patch = false;
     const unsigned tx = nblk(a.g.nx_, kATileX), ty = nblk(rows, kATileY);
     // UpdateRotationMatrizes from the previous moments, before the stream
     launch_rotation_update32(a.g, a.mom, a.ang_old, const_cast<double *>(a.ang_new), s);
@@ -774,7 +775,8 @@ void launch_step_prec_adaptive(const PrecStepArgs &a, const DirTable &dt, bool c
     {
         const size_t smem = apatch_smem(a.nd, a.ng, a.nf);
         const unsigned tiles_x = nblk(a.g.nx_, kAPatchX), tiles_y = nblk(rows, kAPatchY);
-        if (smem <= kAPatchMaxSmem && tiles_x * tiles_y >= kAPatchMinTiles)
+        patch = smem <= kAPatchMaxSmem && tiles_x * tiles_y >= kAPatchMinTiles;
+        if (patch)
             for (unsigned first = 0; first < tiles_y; first += kMaxGridY) // (the grid's y holds so many)
             {
                 PrecStepArgs part = a;
@@ -797,6 +799,7 @@ void launch_step_prec_adaptive(const PrecStepArgs &a, const DirTable &dt, bool c
     }
     // the halo moments, which the reference recomputes from unwritten (zero) intensities
     launch_zero_halo_moments32(a.g, a.mom, s);
+    return patch;
 }
 
 } // namespace grlbm

@@ -1209,9 +1209,9 @@ cudaError_t block_occupancy32(bool curved, int run, int smem, int *blocks)
     return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks, block_kernel32(curved, run, false), block::kThreads, smem);
 }
 
-void launch_step_block32(const Step32Args &a, const BlockStep &b, const DirTable *dt, bool curved, cudaStream_t s)
+int launch_step_block32(const Step32Args &a, const BlockStep &b, const DirTable *dt, bool curved, cudaStream_t s)
 {
-    block::launch_tiles(block_kernel32(curved, b.run, false), block_kernel32(curved, b.run, true), a, b, dt, s);
+    return block::launch_tiles(block_kernel32(curved, b.run, false), block_kernel32(curved, b.run, true), a, b, dt, s);
 }
 
 void launch_step_batch32(const Batch32Item *items, const int *first_tile, int n_items, int total_tiles, int flip,

@@ -866,9 +866,9 @@ cudaError_t block_occupancy64(bool curved, int run, int smem, int *blocks)
     return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks, block_kernel64(curved, run, false), block::kThreads, smem);
 }
 
-void launch_step_block64(const Step64Args &a, const BlockStep &b, const DirTable64 *dt, bool curved, cudaStream_t s)
+int launch_step_block64(const Step64Args &a, const BlockStep &b, const DirTable64 *dt, bool curved, cudaStream_t s)
 {
-    block::launch_tiles(block_kernel64(curved, b.run, false), block_kernel64(curved, b.run, true), a, b, dt, s);
+    return block::launch_tiles(block_kernel64(curved, b.run, false), block_kernel64(curved, b.run, true), a, b, dt, s);
 }
 
 void launch_step64(const Step64Args &a, const DirTable64 *dt, bool curved, int P, int blocks, cudaStream_t s)

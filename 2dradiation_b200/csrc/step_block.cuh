@@ -435,16 +435,17 @@ __global__ void __launch_bounds__(kThreads, F::kMinBlocks)
 
 // Launches the kernel over the step's tiles: `share` on a grid of b.grid
 // blocks where that is fewer than the tiles, else one block a tile: rows of
-// tiles lie along the grid's y, as many at a time as that may hold.
+// tiles lie along the grid's y, as many at a time as that may hold.  Returns
+// the blocks launched.
 template <class Args, class Table>
-void launch_tiles(const void *kernel, const void *share, const Args &a, const BlockStep &b, const Table *dt,
+int launch_tiles(const void *kernel, const void *share, const Args &a, const BlockStep &b, const Table *dt,
                   cudaStream_t s)
 {
     if (b.grid > 0 && b.grid < (int64_t)b.tiles_x * b.tiles_y)
     {
         void *args[] = {const_cast<Args *>(&a), const_cast<BlockStep *>(&b), &dt};
         cudaLaunchKernel(share, dim3(b.grid), dim3(kThreads), args, (size_t)b.smem, s);
-        return;
+        return b.grid;
     }
     for (int first = 0; b.tiles_x > 0 && first < b.tiles_y; first += kMaxGridY)
     {
@@ -454,6 +455,7 @@ void launch_tiles(const void *kernel, const void *share, const Args &a, const Bl
         cudaLaunchKernel(kernel, dim3(b.tiles_x, std::min(b.tiles_y - first, kMaxGridY)), dim3(kThreads), args,
                          (size_t)b.smem, s);
     }
+    return b.tiles_x * b.tiles_y;
 }
 
 // Row stride of the streamed values: 2 modulo the banks (of T), so that the

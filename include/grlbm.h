@@ -311,6 +311,22 @@ int grlbm_copy_node_rows(grlbm_ctx *ctx, int32_t what, int64_t j_first, int64_t 
  * other contexts. */
 int grlbm_set_tile_shape(grlbm_ctx *ctx, int32_t tile_x, int32_t tile_y);
 int grlbm_get_tile_shape(const grlbm_ctx *ctx, int32_t *tile_x, int32_t *tile_y);
+/* No counterpart in the reference.  Which kernel the step last enqueued for
+ * the context runs (alone or in a batch's concurrent launches; a step replayed
+ * from a graph was enqueued when the graph was captured): 0 before the first.
+ * *detail: GRLBM_STEP_BLOCK, the cells of a warp's run (8 or 4);
+ * GRLBM_STEP_PLAIN, whether its collide keeps the streamed values in shared
+ * memory (bit 0) and is the one for a moving or anisotropic fluid (bit 1);
+ * GRLBM_STEP_ADAPTIVE_FP32, 1 where its stream reads a staged patch.  *blocks:
+ * the grid of the first two kernels. */
+enum
+{
+    GRLBM_STEP_BLOCK = 1,     /* the tiled forms, one patch per block */
+    GRLBM_STEP_WARP_TILE = 2, /* the tiled forms, warps with a tile each */
+    GRLBM_STEP_PLAIN = 3,
+    GRLBM_STEP_ADAPTIVE_FP32 = 4
+};
+int grlbm_selftest_step_kernel(const grlbm_ctx *ctx, int32_t *kernel, int32_t *detail, int32_t *blocks);
 /* The most node rows away from its cell that any stream gather reads: the
  * ghost depth a band needs on each side.  From the departure records of the
  * last table build (curved fixed streaming); from the stencil (flat fixed);

@@ -2,7 +2,6 @@
 forms' grids are cut to their shares, a block then takes many tiles, and the
 results are the bits of the problems' own steps."""
 import importlib
-import json
 
 import numpy as np
 import pytest
@@ -27,27 +26,22 @@ def _case(nx, ny, nd, curved=True, moving=False):
     return c
 
 
-def _blocks(problems, shape, path):
-    """Blocks of each step kernel that one batch step launches."""
-    from torch.profiler import ProfilerActivity, profile
+def _kernels(problems, shape):
+    """The kernel and grid of each problem's step in a batch step."""
     with grlbm.Batch(problems) as b:
         b.set_shape(shape)
         b.step(1)
-        with profile(activities=[ProfilerActivity.CUDA]) as p:
-            b.step(1)
-    p.export_chrome_trace(str(path))
-    events = [e for e in json.loads(path.read_text())["traceEvents"] if e.get("cat") == "kernel" and "k_step" in e["name"]]
-    return [int(np.prod(e["args"]["grid"])) for e in events]
+    return [r.step_kernel() for r in problems]
 
 
 @pytest.mark.parametrize("form", ["fp32", "fast64"])
-def test_grids_are_cut_to_the_shares(form, tmp_path):
+def test_grids_are_cut_to_the_shares(form):
     import torch
     sms = torch.cuda.get_device_properties(0).multi_processor_count
     probs = [grlbm.prepare(_case(248, 240, 32), FORMS[form]) for _ in range(2)]
     try:
-        whole = _blocks(probs, 0, tmp_path / "whole.json")
-        share = _blocks(probs, -1, tmp_path / "share.json")
+        whole = [k["blocks"] for k in _kernels(probs, 0)]
+        share = [k["blocks"] for k in _kernels(probs, -1)]
     finally:
         for r in probs:
             r.close()

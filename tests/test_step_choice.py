@@ -3,8 +3,6 @@ up to a number of cells that depends on the form and the directions, warps with
 a tile each from there on, both for the rows of each launch -- and the same
 bits on either side, whole or in bands of rows."""
 import importlib
-import json
-import re
 
 import numpy as np
 import pytest
@@ -32,17 +30,12 @@ def _case(nx, ny, nd, curved, moving=False, cfl=0.9):
     return c
 
 
-def _kernels(step, path):
-    """The step kernels `step` launches: 8 or 4, the cells of a run of the
-    one-patch-per-block kernel, or "warp"."""
-    from torch.profiler import ProfilerActivity, profile
+def _kernel(r, step):
+    """What the step that `step` enqueues last runs: 8 or 4, the cells of a run
+    of the one-patch-per-block kernel, or "warp"."""
     step()
-    with profile(activities=[ProfilerActivity.CUDA]) as p:
-        step()
-    p.export_chrome_trace(str(path))
-    names = [e["name"] for e in json.loads(path.read_text())["traceEvents"] if e.get("cat") == "kernel" and "k_step" in e["name"]]
-    run = [re.search(r"k_step_block<.*, (?:true|false), (\d), (?:true|false)>", n) for n in names]
-    return [int(m[1]) if m else "warp" for m in run]
+    k = r.step_kernel()
+    return k["detail"] if k["kernel"] == "block" else k["kernel"]
 
 
 def _result(r, I0, steps=2):
@@ -63,18 +56,17 @@ def _result(r, I0, steps=2):
     ("fp32", True, 20, 400, 400, False), ("fp32", True, 28, 346, 346, False), ("fp32", True, 28, 347, 347, True),
     ("fast64", True, 32, 316, 316, False), ("fast64", True, 32, 317, 317, True),
     ("fast64", True, 24, 400, 400, False), ("fast64", True, 33, 400, 400, False), ("fast64", False, 32, 600, 600, False)])
-def test_choice_and_bits(form, curved, nd, nx, ny, warp, tmp_path):
+def test_choice_and_bits(form, curved, nd, nx, ny, warp):
     case = _case(nx, ny, nd, curved)
     with grlbm.prepare(case, FORMS[form]) as r:
-        assert _kernels(lambda: r.step(1), tmp_path / "a.json") == (["warp"] if warp else [8])
+        assert _kernel(r, lambda: r.step(1)) == ("warp" if warp else 8)
         # a third of the rows at a time: the block step
         third = 1 + ny // 3
-        rows = lambda: (r.step_rows_async(1, 1 + third, False), r.step_rows_async(1 + third, 1 + ny, True), r.sync())
-        assert _kernels(rows, tmp_path / "b.json")[0] == 8
+        assert _kernel(r, lambda: r.step_rows_async(1, 1 + third, True)) == 8
         # an edge row: runs of 4 up to one 8-cell tile for every second SM
         sms = torch.cuda.get_device_properties(0).multi_processor_count
-        assert _kernels(lambda: (r.step_rows_async(1, 2, True), r.sync()), tmp_path / "c.json") == [
-            4 if 2 * -(-nx // 8) <= sms else 8]
+        assert _kernel(r, lambda: r.step_rows_async(1, 2, True)) == (4 if 2 * -(-nx // 8) <= sms else 8)
+        r.sync()
         I0 = np.random.default_rng(nd).uniform(0.0, 2.0, case["fields"]["eta"].size * nd)
         whole = _result(r, I0, 1)
         r.set_intensity(I0)
@@ -92,14 +84,14 @@ def test_choice_and_bits(form, curved, nd, nx, ny, warp, tmp_path):
 @pytest.mark.parametrize("curved", [False, True])
 @pytest.mark.parametrize("form", ["fp32", "fast64"])
 @pytest.mark.parametrize("nx,ny,nd", [(101, 67, 17), (77, 83, 33), (91, 70, 50), (99, 75, 64)])
-def test_runs_of_eight(form, nx, ny, nd, curved, moving, tmp_path):
+def test_runs_of_eight(form, nx, ny, nd, curved, moving):
     case = _case(nx, ny, nd, curved, moving)
     I0 = np.random.default_rng(7).uniform(0.0, 2.0, case["fields"]["eta"].size * nd)
     with grlbm.prepare(case, FORMS[form]) as r:
-        assert _kernels(lambda: r.step(1), tmp_path / "a.json") == [8]
+        assert _kernel(r, lambda: r.step(1)) == 8
         got = _result(r, I0, 4)
         r.set_tile_shape(2, 1)
-        assert _kernels(lambda: r.step(1), tmp_path / "b.json") == ["warp"]
+        assert _kernel(r, lambda: r.step(1)) == "warp"
         want = _result(r, I0, 4)
     for a, b in zip(got, want):
         assert np.array_equal(a, b)
@@ -107,11 +99,11 @@ def test_runs_of_eight(form, nx, ny, nd, curved, moving, tmp_path):
 
 @pytest.mark.parametrize("curved", [False, True])
 @pytest.mark.parametrize("form", ["fp32", "fast64"])
-def test_far_departures_in_runs_of_eight(form, curved, tmp_path):
+def test_far_departures_in_runs_of_eight(form, curved):
     case = _case(90, 81, 36, curved, cfl=1.8)
     I0 = np.random.default_rng(8).uniform(0.0, 2.0, case["fields"]["eta"].size * 36)
     with grlbm.prepare(case, FORMS[form]) as r:
-        assert _kernels(lambda: r.step(1), tmp_path / "a.json") == [8]
+        assert _kernel(r, lambda: r.step(1)) == 8
         got = _result(r, I0, 4)
         r.set_tile_shape(4, 2)
         want = _result(r, I0, 4)
