@@ -51,6 +51,31 @@ def test_grids_are_cut_to_the_shares(form):
     assert all(x < y for x, y in zip(share, whole)), (whole, share)
 
 
+@pytest.mark.parametrize("shape", [0, -4])
+def test_large_problems_keep_the_block_step(shape):
+    """A problem that runs the warp-per-tile kernel when it has the GPU to
+    itself (512^2 x 16 flat) runs the block step in a batch; the same bits."""
+    case = _case(512, 512, 16, curved=False)
+    I0 = np.random.default_rng(0).uniform(0.0, 2.0, case["fields"]["eta"].size * 16)
+    probs = [grlbm.prepare(case, grlbm.PRECISION_FP32) for _ in range(2)]
+    try:
+        assert all(k["kernel"] == "block" for k in _kernels(probs, shape))
+        probs[0].step(1)
+        assert probs[0].step_kernel()["kernel"] == "warp"
+        for r in probs:
+            r.set_intensity(I0)
+        with grlbm.Batch(probs) as b:
+            b.set_shape(shape)
+            b.step(2)
+        got = probs[0].intensity()
+        probs[1].set_intensity(I0)
+        probs[1].step(2)
+        assert np.array_equal(got, probs[1].intensity())
+    finally:
+        for r in probs:
+            r.close()
+
+
 # grids of many tiles a block, ragged at both edges; every store width and
 # both run lengths (200 directions: runs of 4); a moving fluid
 @pytest.mark.parametrize("shape", [-1, -2])
