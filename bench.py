@@ -213,8 +213,8 @@ def table_build_line(fp32):
     out = {"ms": ms, "rk_substeps": fp32["rk_substeps"], "fp64_flop": flop,
            "achieved_fp64_tflops": flop / (ms * 1e-3) / 1e12 if flop and ms > 0 else None,
            "fp64_peak_tflops_nominal": FP64_PEAK_TFLOPS_NOMINAL,
-           "note": "k_geodesic + k_fourier_project + k_departure, CUDA events; FP64 operations from the committed "
-                   "ncu count of k_geodesic (built without contraction, as the reference rounds)"}
+           "note": "k_geodesic (with the Fourier projection) + k_departure, CUDA events; FP64 operations from the "
+                   "committed ncu count of k_geodesic (contracted multiply-adds)"}
     if out["achieved_fp64_tflops"]:
         out["fp64_frac_nominal"] = out["achieved_fp64_tflops"] / FP64_PEAK_TFLOPS_NOMINAL
     return out
